@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kThreads, 1) replay_map_kernel(
   auto bar = [&](int i) { return bar0 + 8u * static_cast<uint32_t>(i); };
   volatile int* abort_flag = &ctl->abort_flag;
 
-  const int warp = threadIdx.x / 32;
+  const int warp = ptx::warp_index();
   const int lane = threadIdx.x % 32;
   const int qt = blockIdx.x;
   const int bh = blockIdx.y;
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, 1) replay_map_kernel(
   const uint32_t tmem = ctl->tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       ptx::mbar_expect_tx(bar(kQFull), kTileBytes);
       for (int c = 0; c < kChunks; ++c) ptx::tma_load_3d(sQ + c * kChunkBytes, &tm_q, bar(kQFull), c * 64, qrow0, bh);
       // two key tiles (one N = 256 operand) share a barrier pair: the issuing thread pays one wait and one
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, 1) replay_map_kernel(
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       bool ok = ptx::mbar_wait(bar(kQReady), 0, abort_flag);
       if (!ok) report(status, 2, 1, -1);
       const uint64_t dq0 = ptx::smem_desc_sw128(sQ, 16, 1024);

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
   auto bar = [&](int i) { return bar0 + 8u * static_cast<uint32_t>(i); };
   volatile int* abort_flag = &ctl->abort_flag;
 
-  const int warp = threadIdx.x / 32;
+  const int warp = ptx::warp_index();
   const int lane = threadIdx.x % 32;
   // grid: x = work item (mask head, query-tile pair), y = batch.  Blocks start in increasing blockIdx.x;
   // `order` (from the work-list builder) puts long lists first, otherwise items run head by head.
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
   else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       ptx::mbar_expect_tx(bar(kQFull), (has_b ? 2u : 1u) * kTileBytes);
       for (int x = 0; x < (has_b ? 2 : 1); ++x)
         for (int c = 0; c < kChunks; ++c)
@@ -195,19 +195,17 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       // Descriptor bases are built once; inside the loops an MMA costs one 32-bit add per operand (the
       // issuing thread shares its scheduler with two busy softmax warps, so every instruction counts).
-      const uint64_t dq[2] = {ptx::smem_desc_sw128(sQ, 16, 1024), ptx::smem_desc_sw128(sQ + kTileBytes, 16, 1024)};
-      const uint64_t dk[2] = {ptx::smem_desc_sw128(sK, 16, 1024), ptx::smem_desc_sw128(sK + kTileBytes, 16, 1024)};
-      const uint64_t dv[2] = {ptx::smem_desc_sw128(sV, kChunkBytes, 1024),
-                              ptx::smem_desc_sw128(sV + kTileBytes, kChunkBytes, 1024)};
+      const uint64_t dq0 = ptx::smem_desc_sw128(sQ, 16, 1024), dk0 = ptx::smem_desc_sw128(sK, 16, 1024);
+      const uint64_t dv0 = ptx::smem_desc_sw128(sV, kChunkBytes, 1024);
       auto advance = [](uint64_t desc, uint32_t bytes) -> uint64_t {
         // the start-address field (bits 0-13, units of 16 bytes) never carries out for shared-memory addresses
         return (desc & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(desc) + (bytes >> 4));
       };
       auto issue_qk = [&](int x, int s) {
-        const uint64_t a0 = dq[x], b0 = dk[s];
+        const uint64_t a0 = advance(dq0, x * kTileBytes), b0 = advance(dk0, s * kTileBytes);
         const uint32_t d = tmem + x * 128;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
@@ -218,7 +216,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
       };
       // P*V for one half of the key tile (keys [64*half, 64*half+64))
       auto issue_pv_half = [&](int x, int s, int half, uint32_t acc) {
-        const uint64_t b0 = dv[s];
+        const uint64_t b0 = advance(dv0, s * kTileBytes);
         const uint32_t d = tmem + 256 + x * D, a = tmem + x * 128;
 #pragma unroll
         for (int kq = 0; kq < kTile / 32; ++kq) {
@@ -582,7 +580,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
   auto bar = [&](int i) { return bar0 + 8u * static_cast<uint32_t>(i); };
   volatile int* abort_flag = &ctl->abort_flag;
 
-  const int warp = threadIdx.x / 32;
+  const int warp = ptx::warp_index();
   const int lane = threadIdx.x % 32;
   const int npairs = static_cast<int>(gridDim.x) / Hm;
   const int item = order ? order[blockIdx.x] : static_cast<int>(blockIdx.x);
@@ -626,7 +624,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
-      if (lane == 0) {
+      if (ptx::elect_one()) {
         ptx::mbar_expect_tx(bar(k6QFull), (has_b ? 2u : 1u) * kTileBytes);
         for (int x = 0; x < (has_b ? 2 : 1); ++x)
           ptx::tma_load_3d(sQ + x * kTileBytes, &tm_q, bar(k6QFull), 0, (2 * pair + x) * kTile, bh);
@@ -663,7 +661,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
       }
     } else if (warp == 1 || warp == 3) {
       // ------------------------------------------------------------------ MMA issuers, one per query tile
-      if (lane == 0) {
+      if (ptx::elect_one()) {
         const int x = warp >> 1;
         const uint64_t dqx = ptx::smem_desc_sw128(sQ + x * kTileBytes, 16, 1024);
         const uint64_t dk0 = ptx::smem_desc_sw128(sK, 16, 1024);
