@@ -192,15 +192,15 @@ int moddit_solve(const float* mts, const void* factor, int H, int n, int blocks_
                  double regularization, float* X, void* workspace, size_t workspace_bytes, void* stream);
 
 /* The same solve for small systems in the form the specification words it: the normal equations M^T M + reg*I
- * (3n x 3n, float32, closed form) are built in one CTA's shared memory and Cholesky-factored there
+ * (3n x 3n, closed form) are built in one CTA's shared memory and inverted there in float64
  * (moddit_solve_small_prepare, once per (n, blocks_per_frame, reg): the reference caches its factor the same way,
- * MoD/mod/cuda_lstsq.py:153-186); per call the factor is brought into shared memory and one warp per head runs the
- * forward and back substitution for that head's right-hand side (moddit_solve_small).  Float32 arithmetic like the
- * reference's torch.linalg.cholesky + torch.cholesky_solve on the same system (:177,203); no workspace.
+ * MoD/mod/cuda_lstsq.py:153-186); per call every unknown is the dot product of a row of that inverse with the head's
+ * right-hand side, summed in float64 (moddit_solve_small).  It solves the system of the reference's
+ * torch.linalg.cholesky + torch.cholesky_solve (:177,203); no workspace.
  * Limited to n <= moddit_solve_small_max_n() (3n = 224 unknowns fit shared memory; the first configuration of the
  * specification has n = 64); larger n return MODDIT_E_UNSUPPORTED - use moddit_solve_prepare + moddit_solve, whose
  * structured elimination has no such limit.
- *   factor : moddit_solve_small_factor_bytes(n) bytes (the lower-triangular factor, (3n)^2 float32)
+ *   factor : moddit_solve_small_factor_bytes(n) bytes (the inverse: (3n)^2 float32 values, then their remainders)
  *   mts    : (H, 3n) float32      X : (H, 3n) float32, same unknown order as moddit_solve */
 int moddit_solve_small_max_n(void);
 size_t moddit_solve_small_factor_bytes(int n);

@@ -190,86 +190,79 @@ __global__ void mtm_kernel(int n, int bpf, float reg, float* __restrict__ mtm) {
   mtm[idx] = mtm_entry(static_cast<int>(idx / F), static_cast<int>(idx % F), n, bpf, reg);
 }
 
-// ---- small systems: normal equations in shared memory, Cholesky, one warp per head -------------------------------
-// For 3n <= kSmallMaxF unknowns the whole Gram matrix fits one CTA's shared memory in float32 (rows padded by one
-// word so that column walks do not collide on a bank).  `solve_small_factor_kernel` (once per geometry, like the
-// reference's cached factor, MoD/mod/cuda_lstsq.py:153-186) builds it from the closed form and factors it in place
-// (right-looking Cholesky, a warp per row of the trailing update); `solve_small_kernel` (per call) brings the
-// factor into shared memory and every warp takes the right-hand side of one head: forward and back substitution
-// as warp-wide dot products, float32 like the reference's torch.linalg.cholesky / cholesky_solve on this system
-// (MoD/mod/cuda_lstsq.py:177,203).
+// ---- small systems: inverse of the normal equations, one dot product per unknown ---------------------------------
+// For 3n <= kSmallMaxF unknowns the lower triangle of the Gram matrix fits one CTA's shared memory in float64.
+// `solve_small_factor_kernel` (once per geometry, like the reference's cached factor, MoD/mod/cuda_lstsq.py:153-186)
+// builds it from the closed form and inverts it there with the symmetric sweep: after sweeping every pivot the matrix
+// holds -(M^T M + reg I)^-1.  Each element of the inverse is kept as two float32 words (value, remainder).
+// `solve_small_kernel` (per call) is then a matrix-vector product per head, float64 sums, a warp per unknown.
+// Bound: latency.  Forward and back substitution with a float32 Cholesky factor, a warp per head, is a chain of 2 * 3n
+// dot products that each wait for the one before: 147 us at n = 64, where the product is one load deep.
 constexpr int kSmallMaxF = 224;
 constexpr int kSmallFactorThreads = 1024;
 constexpr int kSmallThreads = 256;
+constexpr int kSmallHeads = 4;      // heads per warp: a word of the inverse is loaded once for all of them
+
+__device__ __forceinline__ int tri(int i, int j) { return i >= j ? i * (i + 1) / 2 + j : j * (j + 1) / 2 + i; }
 
 __global__ void __launch_bounds__(kSmallFactorThreads) solve_small_factor_kernel(int n, int bpf, float reg,
-                                                                                float* __restrict__ L) {
-  extern __shared__ __align__(16) float small_smem[];
+                                                                                float* __restrict__ inv) {
+  extern __shared__ __align__(16) double small_tri[];    // lower triangle, rows one after the other
   const int F = 3 * n;
-  const int ld = F + 1;
-  float* A = small_smem;                                 // [F][ld], lower triangle becomes L
+  double* col = small_tri + static_cast<size_t>(F) * (F + 1) / 2;        // column of the pivot before the sweep
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  for (int e = tid; e < F * F; e += kSmallFactorThreads) {
-    const int a = e / F, b = e - a * F;
-    A[a * ld + b] = mtm_entry(a, b, n, bpf, reg);
-  }
+  for (int i = warp; i < F; i += kSmallFactorThreads / 32)
+    for (int j = lane; j <= i; j += 32) small_tri[tri(i, j)] = static_cast<double>(mtm_entry(i, j, n, bpf, reg));
   __syncthreads();
   for (int k = 0; k < F; ++k) {
-    const float piv = sqrtf(A[k * ld + k]);              // every thread reads the same word; thread 0 writes it below
+    for (int i = tid; i < F; i += kSmallFactorThreads) col[i] = small_tri[tri(i, k)];
     __syncthreads();
-    if (tid == 0) A[k * ld + k] = piv;
-    const float inv = 1.0f / piv;
-    for (int i = k + 1 + tid; i < F; i += kSmallFactorThreads) A[i * ld + k] *= inv;
-    __syncthreads();
-    // trailing update of the lower triangle: A[i][j] -= L[i][k] * L[j][k] for k < j <= i; a warp per row
-    for (int i = k + 1 + warp; i < F; i += kSmallFactorThreads / 32) {
-      const float lik = A[i * ld + k];
-      for (int j = k + 1 + lane; j <= i; j += 32) A[i * ld + j] = fmaf(-lik, A[j * ld + k], A[i * ld + j]);
+    const double p = 1.0 / col[k];
+    for (int i = warp; i < F; i += kSmallFactorThreads / 32) {
+      const double ci = col[i] * p;
+      for (int j = lane; j <= i; j += 32) {
+        double& a = small_tri[tri(i, j)];
+        if (i == k && j == k) a = -p;
+        else if (i == k) a = col[j] * p;
+        else if (j == k) a = ci;
+        else a = fma(-ci, col[j], a);
+      }
     }
     __syncthreads();
   }
   for (int e = tid; e < F * F; e += kSmallFactorThreads) {
-    const int a = e / F, b = e - a * F;
-    L[e] = (b <= a) ? A[a * ld + b] : 0.f;
+    const double v = -small_tri[tri(e / F, e % F)];
+    const float hi = static_cast<float>(v);
+    inv[e] = hi;
+    inv[F * F + e] = static_cast<float>(v - static_cast<double>(hi));
   }
 }
 
 __global__ void __launch_bounds__(kSmallThreads) solve_small_kernel(const float* __restrict__ mts,
-                                                                    const float* __restrict__ L, int H, int n,
+                                                                    const float* __restrict__ inv, int H, int n,
                                                                     float* __restrict__ X) {
-  extern __shared__ __align__(16) float small_smem[];
   const int F = 3 * n;
-  const int ld = F + 1;
-  float* A = small_smem;                                 // [F][ld]: the factor
-  float* ys = A + static_cast<size_t>(F) * ld;           // [warps][F] right-hand sides / solutions
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  for (int e = tid; e < F * F; e += kSmallThreads) {
-    const int a = e / F, b = e - a * F;
-    A[a * ld + b] = L[e];
-  }
-  __syncthreads();
-  const int h = blockIdx.x * (kSmallThreads / 32) + warp;
-  if (h >= H) return;                                     // no block-wide barrier below this line
-  float* y = ys + warp * F;
-  for (int i = lane; i < F; i += 32) y[i] = mts[static_cast<int64_t>(h) * F + i];
-  __syncwarp();
-  for (int i = 0; i < F; ++i) {                           // L y = b
-    float acc = 0.f;
-    for (int j = lane; j < i; j += 32) acc = fmaf(A[i * ld + j], y[j], acc);
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int i = blockIdx.y * (kSmallThreads / 32) + warp;
+  if (i >= F) return;
+  const int h0 = blockIdx.x * kSmallHeads;
+  double acc[kSmallHeads] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) y[i] = (y[i] - acc) / A[i * ld + i];
-    __syncwarp();
-  }
-  for (int i = F - 1; i >= 0; --i) {                      // L^T x = y
-    float acc = 0.f;
-    for (int j = i + 1 + lane; j < F; j += 32) acc = fmaf(A[j * ld + i], y[j], acc);
+  for (int u = 0; u < kSmallMaxF / 32; ++u) {            // all loads of the row in flight at once
+    const int j = lane + 32 * u;
+    if (j < F) {
+      const double a = static_cast<double>(__ldg(inv + i * F + j)) + static_cast<double>(__ldg(inv + F * F + i * F + j));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) y[i] = (y[i] - acc) / A[i * ld + i];
-    __syncwarp();
+      for (int hh = 0; hh < kSmallHeads; ++hh)
+        if (h0 + hh < H) acc[hh] = fma(a, static_cast<double>(__ldg(mts + static_cast<int64_t>(h0 + hh) * F + j)), acc[hh]);
+    }
   }
-  for (int i = lane; i < F; i += 32) X[static_cast<int64_t>(h) * F + i] = y[i];
+#pragma unroll
+  for (int hh = 0; hh < kSmallHeads; ++hh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[hh] += __shfl_xor_sync(0xffffffffu, acc[hh], o);
+    if (lane == 0 && h0 + hh < H) X[static_cast<int64_t>(h0 + hh) * F + i] = static_cast<float>(acc[hh]);
+  }
 }
 
 // ---- solve set-up -------------------------------------------------------------------------------
@@ -741,7 +734,7 @@ extern "C" int moddit_solve(const float* mts, const void* factor, int H, int n, 
 extern "C" int moddit_solve_small_max_n(void) { return kSmallMaxF / 3; }
 
 extern "C" size_t moddit_solve_small_factor_bytes(int n) {
-  return (n > 0 && 3 * n <= kSmallMaxF) ? sizeof(float) * static_cast<size_t>(3 * n) * (3 * n) : 0;
+  return (n > 0 && 3 * n <= kSmallMaxF) ? 2 * sizeof(float) * static_cast<size_t>(3 * n) * (3 * n) : 0;
 }
 
 static int check_small(const char* who, int n) {
@@ -761,7 +754,7 @@ extern "C" int moddit_solve_small_prepare(int n, int blocks_per_frame, float reg
   if (int rc = check_small("solve_small_prepare", n)) return rc;
   if (int rc = require_sm100()) return rc;
   const int F = 3 * n;
-  const size_t smem = sizeof(float) * static_cast<size_t>(F) * (F + 1);
+  const size_t smem = sizeof(double) * (static_cast<size_t>(F) * (F + 1) / 2 + F);
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(solve_small_factor_kernel), smem)) return rc;
   solve_small_factor_kernel<<<1, kSmallFactorThreads, smem, as_stream(stream)>>>(n, blocks_per_frame, regularization,
                                                                                 factor);
@@ -776,9 +769,8 @@ extern "C" int moddit_solve_small(const float* mts, const float* factor, int H, 
   if (int rc = check_small("solve_small", n)) return rc;
   if (int rc = require_sm100()) return rc;
   const int F = 3 * n;
-  const size_t smem = sizeof(float) * (static_cast<size_t>(F) * (F + 1) + static_cast<size_t>(kSmallThreads / 32) * F);
-  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(solve_small_kernel), smem)) return rc;
-  solve_small_kernel<<<ceil_div(H, kSmallThreads / 32), kSmallThreads, smem, as_stream(stream)>>>(mts, factor, H, n, X);
+  solve_small_kernel<<<dim3(ceil_div(H, kSmallHeads), ceil_div(F, kSmallThreads / 32)), kSmallThreads, 0, as_stream(stream)>>>(
+      mts, factor, H, n, X);
   MODDIT_CHECK_LAUNCH("solve_small_kernel");
   return MODDIT_OK;
 }

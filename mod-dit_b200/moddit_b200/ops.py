@@ -431,7 +431,7 @@ def solve_factor(n: int, blocks_per_frame: int, regularization: float, device) -
 
 
 def _small_factor(n: int, blocks_per_frame: int, regularization: float, device) -> torch.Tensor:
-    """Float32 Cholesky factor of the small system, computed once per (device, n, bpf, lambda)."""
+    """Inverse of the small system, computed once per (device, n, bpf, lambda)."""
     device = torch.device(device)
     key = ("small", device.index if device.index is not None else torch.cuda.current_device(), n,
            int(blocks_per_frame), float(regularization))
@@ -454,8 +454,8 @@ def solve(mts_: torch.Tensor, n: int, blocks_per_frame: int, regularization: flo
           method: str = "auto") -> torch.Tensor:
     """X (H, 3n) float32 with (M^T M + regularization * I) X = mts.
 
-    method "small": normal equations in shared memory, float32 Cholesky, one warp per head (`moddit_solve_small`;
-    n <= `lib.moddit_solve_small_max_n()`); "structured": the float64 structured elimination against a factor
+    method "small": normal equations inverted in shared memory once per geometry, one product per call
+    (`moddit_solve_small`; n <= `lib.moddit_solve_small_max_n()`); "structured": the float64 structured elimination against a factor
     cached per geometry (`moddit_solve`); "auto": "small" where it fits and regularization >= 0.5, else
     "structured"."""
     dev = _need_cuda(mts_)
