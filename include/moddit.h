@@ -207,6 +207,11 @@ size_t moddit_solve_small_factor_bytes(int n);
 int moddit_solve_small_prepare(int n, int blocks_per_frame, float regularization, float* factor, void* stream);
 int moddit_solve_small(const float* mts, const float* factor, int H, int n, float* X, void* stream);
 
+/* Raw solution X (H, 3n) -> the features of MoD/mod/cuda_lstsq.py:257-261: d (H, 2n-1), c (H, n) halved, b_d (H),
+ * all float32, and, unless modes is NULL, the per-head mode of moddit_head_modes for `threshold`. */
+int moddit_split_solution(const float* X, int H, int n, float threshold, float* d, float* c, float* b_d,
+                          int32_t* modes, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Line selection.  Replaces `choose_topk_lines` (MoD/mod/attn_mask.py:351-370): extrapolate
  * cur + (cur-last)/predict_T for verticals c (H,n) and diagonals d (H,2n-1), concatenate [c | d],

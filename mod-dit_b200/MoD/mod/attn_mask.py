@@ -602,7 +602,7 @@ def _pooled_step(query, key, value, warmup_state, logger, pre_defined_mask, curr
     n = dark.shape[-1]
     mts, _ = _ops.mts(dark, warmup_state['blocks_per_frame'])
     X = _ops.solve(mts, n, warmup_state['blocks_per_frame'], 1.0)
-    feats = features_from_solution(X, n)
+    feats, modes = _ops.split_solution(X, n, 1.0)                 # device-side modes: no host sync per step
     history = warmup_state.get('features_history') or []
     if current_step == warmup_steps - 2 or not history:
         warmup_state['features_history'] = [feats]
@@ -617,7 +617,7 @@ def _pooled_step(query, key, value, warmup_state, logger, pre_defined_mask, curr
     warmup_state['features_history'] = history
     warmup_state['current_steps'] = current_step + 1
     warmup_state['prev_full_maps'] = dark
-    warmup_state['mode'] = _ops.head_modes(feats['b_d'], 1.0)     # device-side modes: no host sync per step
+    warmup_state['mode'] = modes
     mask = _select_and_build(warmup_state, num_heads, seq_len, query.device, dark_map=dark)
     _store_mask(warmup_state, mask, seq_len)
     output = AttentionSparseEngine(query, key, value, mask, pre_defined_mask=pre_defined_mask,

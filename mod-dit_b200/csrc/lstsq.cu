@@ -616,6 +616,42 @@ __global__ void __launch_bounds__(256) reconstruct_map_kernel(const float* __res
 }  // namespace
 }  // namespace moddit
 
+namespace moddit {
+namespace {
+// Raw solution (H, 3n) -> features: diagonals, halved columns, block coefficient, and the head's mode from the latter.
+// Launch-bound (n = 64: 1.5 us); as slices and a division of the tensor library it was four copies and a launch for the
+// modes, each with its own gap (1.4 - 2.8 us each).
+__global__ void __launch_bounds__(256) split_solution_kernel(const float* __restrict__ X, int H, int n, float threshold,
+                                                             float* __restrict__ d, float* __restrict__ c,
+                                                             float* __restrict__ b_d, int32_t* __restrict__ modes) {
+  const int h = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x;
+  const int nd = 2 * n - 1;
+  if (i >= 3 * n) return;
+  const float x = X[static_cast<int64_t>(h) * 3 * n + i];
+  if (i < nd) {
+    d[static_cast<int64_t>(h) * nd + i] = x;
+  } else if (i < nd + n) {
+    c[static_cast<int64_t>(h) * n + (i - nd)] = x / 2.f;
+  } else {
+    b_d[h] = x;
+    if (modes != nullptr) modes[h] = (x <= threshold) ? MODDIT_MODE_BLOCK_DIAGONAL : MODDIT_MODE_SPARSE;
+  }
+}
+}  // namespace
+}  // namespace moddit
+
+extern "C" int moddit_split_solution(const float* X, int H, int n, float threshold, float* d, float* c, float* b_d,
+                                     int32_t* modes, void* stream) {
+  clear_error();
+  MODDIT_CHECK_ARG(X && d && c && b_d, "split_solution: null pointer");
+  MODDIT_CHECK_ARG(H > 0 && H <= 65535, "split_solution: H=%d out of range", H);
+  if (int rc = check_n("split_solution", n)) return rc;
+  if (int rc = require_sm100()) return rc;
+  split_solution_kernel<<<dim3(ceil_div(3 * n, 256), H), 256, 0, as_stream(stream)>>>(X, H, n, threshold, d, c, b_d, modes);
+  MODDIT_CHECK_LAUNCH("split_solution_kernel");
+  return MODDIT_OK;
+}
+
 extern "C" int moddit_reconstruct_map(const float* d, const float* c, const float* b_d, int H, int n,
                                       int blocks_per_frame, float* out, void* stream) {
   clear_error();

@@ -486,6 +486,23 @@ def solve(mts_: torch.Tensor, n: int, blocks_per_frame: int, regularization: flo
     return X
 
 
+def split_solution(X: torch.Tensor, n: int, threshold: float = 1.0):
+    """Raw solution (H, 3n) float32 -> ({'d': (H,2n-1), 'c': (H,n) halved, 'b_d': (H,)}, (H,) int32 modes as `head_modes`
+    gives them for `threshold`), in one launch."""
+    dev = _need_cuda(X)
+    if X.dtype != torch.float32 or X.dim() != 2 or X.shape[1] != 3 * n or not X.is_contiguous():
+        raise ValueError("X must be a contiguous float32 (H, 3n) tensor")
+    H = X.shape[0]
+    d = torch.empty(H, 2 * n - 1, device=dev, dtype=torch.float32)
+    c = torch.empty(H, n, device=dev, dtype=torch.float32)
+    b_d = torch.empty(H, device=dev, dtype=torch.float32)
+    modes = torch.empty(H, device=dev, dtype=torch.int32)
+    with torch.cuda.device(dev), _timed("moddit_split_solution", dev):
+        check(lib.moddit_split_solution(_ptr(X), H, n, float(threshold), _ptr(d), _ptr(c), _ptr(b_d), _ptr(modes),
+                                        _stream(dev)), "moddit_split_solution")
+    return {'d': d, 'c': c, 'b_d': b_d}, modes
+
+
 # ---------------------------------------------------------------------------------------------
 # selection, masks, work lists
 # ---------------------------------------------------------------------------------------------
