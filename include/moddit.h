@@ -284,6 +284,23 @@ int moddit_tile_lists(const uint8_t* mask, int Hm, int nbq, int nbk, int block_s
  */
 int moddit_order_pairs(const int32_t* counts, int Hm, int npairs, int heads_per_group, int32_t* order, void* stream);
 
+/* The stages from moddit_pool_blocks to moddit_tile_lists in one call, for a step that predicts its mask from this
+ * step's q and k (the pooled producer) and the features of the step before; every output equals what the single entry
+ * points give.
+ *   first, n  : video region in blocks: blocks [first, first + n) of ceil(N / block_size)
+ *   factor    : from moddit_solve_small_prepare (small_solve != 0) or moddit_solve_prepare, regularization 1
+ *   last_c/d  : features of the step before; d, c, b_d, modes, map_f16 receive this step's
+ *   mask, counts, entries, order : as moddit_mask_from_lines / moddit_tile_lists write them
+ *   workspace : moddit_predict_workspace_bytes(...) bytes of scratch, 16-byte aligned
+ */
+size_t moddit_predict_workspace_bytes(int H, int nb, int D, int n, int top_k, int small_solve);
+int moddit_predict_lines(const void* q, const void* k, int dtype, int H, int N, int D, int block_size, int first,
+                         int n, int blocks_per_frame, int mask_layout, float scale, const void* factor,
+                         int small_solve, const float* last_c, const float* last_d, int top_k, float predict_T,
+                         float mode_threshold, void* map_f16, float* d, float* c, float* b_d, int32_t* modes,
+                         uint8_t* mask, int32_t* counts, int32_t* entries, int32_t* order, void* workspace,
+                         size_t workspace_bytes, void* stream);
+
 /* Block-sparse flash-attention forward.  Replaces `AttentionSparseEngine` (MoD/mod/attn_mask.py:266-331:
  * block_sparse_sage2_attn_cuda for video rows, flashinfer prefill for text rows, sageattn for all-true
  * masks) and, with all-true lists and `lse` non-null, the dense pass of

@@ -579,6 +579,18 @@ def _spargeattn_step(query, key, value, warmup_state):
     return output, {'mode': 'warmup', 'mask': None}
 
 
+def _predicts_in_one_call(query, warmup_state, history, current_step) -> bool:
+    """Whether a step's prediction is the plain line prediction of one sequence, which is a single call; stages that are
+    being timed one by one, work lists ordered by groups of heads and the other selector go stage by stage."""
+    return (bool(history) and current_step != warmup_state['warmup_steps'] - 2
+            and query.shape[0] == 1 and warmup_state['model_type'] in _lib.LAYOUT
+            and warmup_state.get('selector', 'topk_lines') != 'cumulative_mass'
+            and int(warmup_state.get('_head_groups') or 1) <= 1
+            and tuple(history[-1]['c'].shape) == (query.shape[1], _geometry(warmup_state, query.shape[2])[1])
+            and history[-1]['c'].device == query.device
+            and not _ops.timing_active("moddit_pool_blocks"))
+
+
 def _pooled_step(query, key, value, warmup_state, logger, pre_defined_mask, current_step, layer_idx,
                  value_ready=None, output_scatter=None, pooled_qk=None, qk_ready=None, head_group_ready=None):
     """Variant with the mean-pooled map producer: the mask is re-predicted on every step from the pooled map
@@ -598,12 +610,32 @@ def _pooled_step(query, key, value, warmup_state, logger, pre_defined_mask, curr
     if pooled_qk is None:                               # query and key are read by the pooling itself
         for ev in _events(qk_ready) + _events(head_group_ready):
             torch.cuda.current_stream(query.device).wait_event(ev)
+    history = warmup_state.get('features_history') or []
+    if pooled_qk is None and _predicts_in_one_call(query, warmup_state, history, current_step):
+        _, n, first = _geometry(warmup_state, seq_len)
+        dark, feats, modes, mask, lists = _ops.predict_lines(
+            query, key, bs, first=first, n=n, blocks_per_frame=warmup_state['blocks_per_frame'],
+            model_type=warmup_state['model_type'], last=history[-1], top_k=warmup_state['top_k'],
+            predict_T=warmup_state['predict_T'])
+        history.append(feats)
+        if len(history) > 2:
+            history.pop(0)
+        warmup_state['features_history'] = history
+        warmup_state['current_steps'] = current_step + 1
+        warmup_state['prev_full_maps'] = dark
+        warmup_state['mode'] = modes
+        warmup_state['mask'] = mask
+        warmup_state['_tile_lists'] = (mask, lists)
+        output = AttentionSparseEngine(query, key, value, mask, pre_defined_mask=pre_defined_mask,
+                                       video_token_num=warmup_state.get('video_token_num', 0), block_size=bs,
+                                       _lists=lists, _value_ready=(value_ready, qk_ready), _scatter=output_scatter,
+                                       _group_ready=head_group_ready)
+        return output, {'mask': mask}
     dark = compute_pooled_map(query, key, warmup_state, pooled_qk).squeeze(0)
     n = dark.shape[-1]
     mts, _ = _ops.mts(dark, warmup_state['blocks_per_frame'])
     X = _ops.solve(mts, n, warmup_state['blocks_per_frame'], 1.0)
     feats, modes = _ops.split_solution(X, n, 1.0)                 # device-side modes: no host sync per step
-    history = warmup_state.get('features_history') or []
     if current_step == warmup_steps - 2 or not history:
         warmup_state['features_history'] = [feats]
         warmup_state['current_steps'] = current_step + 1

@@ -29,6 +29,8 @@ KERNELS_PER_CALL = {"moddit_pool_blocks": 1, "moddit_pooled_map": 1, "moddit_poo
                     "moddit_mtm": 1, "moddit_solve": 3, "moddit_select_lines": 1, "moddit_head_modes": 1,
                     "moddit_mask_from_lines": 1, "moddit_select_mass": 1, "moddit_tile_lists": 2,
                     "moddit_sparse_attn_fwd": 1, "moddit_replay_status": 0,
+                    # the stages of a prediction in one call: 2 + 3 + 2 + 3 (1 with the small solve) + 1 + 1 + 1 + 2
+                    "moddit_predict_lines": 15, "moddit_predict_lines (small)": 13,
                     "moddit_mts_noalloc": 2, "moddit_copy_rows_dma": 0, "moddit_qkv_prologue": 1}
 
 
@@ -450,6 +452,12 @@ def _small_factor(n: int, blocks_per_frame: int, regularization: float, device) 
         return fac
 
 
+def _takes_small_solve(n: int, regularization: float) -> bool:
+    """The float32-system route only for well-conditioned systems (the regularisation the path uses is 1; with a tiny
+    one the unregularised rank deficiency is a float32 pivot away)."""
+    return n <= lib.moddit_solve_small_max_n() and regularization >= 0.5
+
+
 def solve(mts_: torch.Tensor, n: int, blocks_per_frame: int, regularization: float,
           method: str = "auto") -> torch.Tensor:
     """X (H, 3n) float32 with (M^T M + regularization * I) X = mts.
@@ -465,9 +473,7 @@ def solve(mts_: torch.Tensor, n: int, blocks_per_frame: int, regularization: flo
     if method not in ("auto", "small", "structured"):
         raise ValueError("method must be 'auto', 'small' or 'structured'")
     H = mts_.shape[0]
-    # "auto" takes the float32 route only for well-conditioned systems (the regularisation the path uses is 1;
-    # with a tiny one the unregularised rank deficiency is a float32 pivot away)
-    if method == "small" or (method == "auto" and n <= lib.moddit_solve_small_max_n() and regularization >= 0.5):
+    if method == "small" or (method == "auto" and _takes_small_solve(n, regularization)):
         if n > lib.moddit_solve_small_max_n():
             raise ValueError(f"solve: 3n = {3 * n} unknowns exceed the {3 * lib.moddit_solve_small_max_n()} that fit "
                              "shared memory; use method='structured'")
@@ -649,6 +655,50 @@ def tile_lists(mask: torch.Tensor, block_size: int, n_tokens: int, kv_block_limi
             check(lib.moddit_order_pairs(_ptr(counts), Hm, npairs, int(heads_per_group), _ptr(order), _stream(dev)),
                   "moddit_order_pairs")
     return TileLists(counts, entries, order)
+
+
+def predict_lines(q: torch.Tensor, k: torch.Tensor, block_size: int, *, first: int, n: int, blocks_per_frame: int,
+                  model_type: str, last: Dict[str, torch.Tensor], top_k: int, predict_T: float, threshold: float = 1.0):
+    """The mask prediction of a step in one call (`moddit_predict_lines`): block means of (1,H,N,D) q and k, pooled map,
+    line fit, features, line selection against the features `last` of the step before, mask, work lists.
+
+    Returns (map (H,n,n) float16, {'d', 'c', 'b_d'}, modes, mask, TileLists), each equal to what `pool_blocks`,
+    `pooled_map`, `mts`, `solve`, `split_solution`, `select_lines`, `mask_from_lines` and `tile_lists` give."""
+    dev = _need_cuda(q, k, last['c'], last['d'])
+    _need_contig(q=q, k=k)
+    if q.shape != k.shape or q.dtype != k.dtype or q.dim() != 4 or q.shape[0] != 1:
+        raise ValueError("query and key must be (1, H, N, D) tensors of one dtype")
+    if model_type not in _lib.LAYOUT:
+        raise ValueError(f"Unknown model_type: {model_type}, expected 'wan', 'hunyuan', or 'cogvideox'")
+    _, H, N, D = q.shape
+    last_c, last_d = (last[key].to(torch.float32).contiguous() for key in ('c', 'd'))
+    if tuple(last_c.shape) != (H, n) or tuple(last_d.shape) != (H, 2 * n - 1):
+        raise ValueError("feature shapes must be c:(H,n) d:(H,2n-1)")
+    nb = (N + block_size - 1) // block_size
+    ntq = (N + 127) // 128
+    npairs = (ntq + 1) // 2
+    nbt = n if model_type == "wan" else nb
+    small = _takes_small_solve(n, 1.0)
+    factor = (_small_factor if small else solve_factor)(n, blocks_per_frame, 1.0, dev)
+    f32 = dict(device=dev, dtype=torch.float32)
+    i32 = dict(device=dev, dtype=torch.int32)
+    dark = torch.empty(H, n, n, device=dev, dtype=torch.float16)
+    d, c, b_d = torch.empty(H, 2 * n - 1, **f32), torch.empty(H, n, **f32), torch.empty(H, **f32)
+    modes = torch.empty(H, **i32)
+    mask = torch.empty(H, nbt, nbt, device=dev, dtype=torch.bool)
+    counts, order = torch.empty(H, npairs, **i32), torch.empty(H, npairs, **i32)
+    entries = torch.empty(H, npairs, ntq, **i32)
+    wsb = lib.moddit_predict_workspace_bytes(H, nb, D, n, int(top_k), int(small))
+    ws = torch.empty(max(wsb, 16), device=dev, dtype=torch.uint8)
+    name = "moddit_predict_lines (small)" if small else "moddit_predict_lines"
+    with torch.cuda.device(dev), _timed(name, dev):
+        check(lib.moddit_predict_lines(
+            q.data_ptr(), k.data_ptr(), _qkv_dtype(q), H, N, D, block_size, int(first), int(n), int(blocks_per_frame),
+            _lib.LAYOUT[model_type], float(D) ** -0.5, factor.data_ptr(), int(small), last_c.data_ptr(), last_d.data_ptr(),
+            int(top_k), float(predict_T), float(threshold), dark.data_ptr(), d.data_ptr(), c.data_ptr(), b_d.data_ptr(),
+            modes.data_ptr(), mask.data_ptr(), counts.data_ptr(), entries.data_ptr(), order.data_ptr(), ws.data_ptr(), wsb,
+            _stream(dev)), "moddit_predict_lines")
+    return dark, {'d': d, 'c': c, 'b_d': b_d}, modes, mask, TileLists(counts, entries, order)
 
 
 def copy_rows(src_ptr: int, dst_ptr: int, src_pitch: int, dst_pitch: int, width_bytes: int, rows: int,
