@@ -44,6 +44,13 @@ int g_optin_count = 0;
 std::mutex g_optin_mutex;
 }  // namespace
 
+int sm_count(int* sms) {
+  int dev = 0;
+  MODDIT_CHECK_CUDA(cudaGetDevice(&dev));
+  MODDIT_CHECK_CUDA(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
+  return MODDIT_OK;
+}
+
 int ensure_dynamic_smem(const void* kernel, size_t bytes) {
   if (bytes <= 48 * 1024) return MODDIT_OK;          // available without opting in
   int dev = 0;

@@ -49,4 +49,7 @@ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // once per call.  Returns MODDIT_OK or a failure code (message set).
 int ensure_dynamic_smem(const void* kernel, size_t bytes);
 
+// Number of SMs of the current device.
+int sm_count(int* sms);
+
 }  // namespace moddit
