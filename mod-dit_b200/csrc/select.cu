@@ -29,7 +29,8 @@ constexpr int kSelectThreads = 1024;
 // One CTA per head: the L = 3n - 1 extrapolated line intensities become 64-bit keys (value order << 32 | index),
 // padded to a power of two P with all-ones keys, and are bitonic-sorted ascending in shared memory; the first k
 // of the order are the selection (smallest value first, equal values lowest index first - the same total order
-// as ranking every element against every other, at L log^2 L instead of L^2 compares).
+// as ranking every element against every other, at L log^2 L instead of L^2 compares).  A thread per pair of keys up to
+// kSelectThreads: the sort is a chain of block-wide barriers, and idle warps only make each of them slower.
 __global__ void __launch_bounds__(kSelectThreads) select_lines_kernel(
     const float* __restrict__ cur_c, const float* __restrict__ cur_d, const float* __restrict__ last_c,
     const float* __restrict__ last_d, int n, int k, int P, float predict_T, int64_t* __restrict__ selected) {
@@ -37,7 +38,7 @@ __global__ void __launch_bounds__(kSelectThreads) select_lines_kernel(
   const int h = blockIdx.x;
   const int nd = 2 * n - 1;
   const int L = n + nd;
-  for (int i = threadIdx.x; i < P; i += kSelectThreads) {
+  for (int i = threadIdx.x; i < P; i += blockDim.x) {
     if (i >= L) {
       sort_keys[i] = ~0ull;
       continue;
@@ -57,7 +58,7 @@ __global__ void __launch_bounds__(kSelectThreads) select_lines_kernel(
   __syncthreads();
   for (int size = 2; size <= P; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = threadIdx.x; t < P / 2; t += kSelectThreads) {
+      for (int t = threadIdx.x; t < P / 2; t += blockDim.x) {
         const int lo = 2 * t - (t & (stride - 1));
         const int hi = lo + stride;
         const bool up = ((lo & size) == 0);
@@ -71,7 +72,7 @@ __global__ void __launch_bounds__(kSelectThreads) select_lines_kernel(
     }
   }
   __syncthreads();
-  for (int r = threadIdx.x; r < k; r += kSelectThreads)
+  for (int r = threadIdx.x; r < k; r += blockDim.x)
     selected[static_cast<int64_t>(h) * k + r] = static_cast<int64_t>(static_cast<uint32_t>(sort_keys[r]));
 }
 
@@ -515,7 +516,8 @@ extern "C" int moddit_select_lines(const float* cur_c, const float* cur_d, const
   while (P < L) P <<= 1;
   const size_t smem = sizeof(unsigned long long) * P;     // at most 128 KB (n <= 4096)
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(select_lines_kernel), smem)) return rc;
-  select_lines_kernel<<<H, kSelectThreads, smem, as_stream(stream)>>>(cur_c, cur_d, last_c, last_d, n, k, P, predict_T,
+  const int threads = P / 2 < 32 ? 32 : (P / 2 < kSelectThreads ? P / 2 : kSelectThreads);
+  select_lines_kernel<<<H, threads, smem, as_stream(stream)>>>(cur_c, cur_d, last_c, last_d, n, k, P, predict_T,
                                                                       selected);
   MODDIT_CHECK_LAUNCH("select_lines_kernel");
   return MODDIT_OK;
