@@ -91,44 +91,11 @@ struct PrologueArgs {
   float eps;
 };
 
-// Grid: x < ceil(H / kHeads): q and k of kHeads heads; then one CTA per head of v; y = token block, z = batch - the CTAs of
-// one token block run together, so the rotary table rows of the block are fetched from HBM once and shared through L2.
+// Grid: x = head + H * tensor (q, k, v), y = token block, z = batch - the CTAs of one token block run together,
+// so the rotary table rows of the block are fetched from HBM once and shared through L2.
 // kRope is the table form (MODDIT_ROPE_*); whether anything is rotated is decided at run time.
-//
-// A CTA rotates its rows in q and k of two heads with table values it reads once: a row's cos and sin are 8 * D bytes
-// in float32, four times the row itself, so with one head of one tensor per CTA the tables were most of what the L2
-// had to deliver (at 24 heads of 128 and 128-row blocks 7.6 GB beside 2.1 GB of rows).
-constexpr int kHeads = 2;
-constexpr int kUnits = 2 * kHeads;          // unit c of a CTA: tensor c & 1 (q, k) of head h0 + c / 2
-
-// The move to head-major layout alone (v).
-template <typename T, int D>
-__device__ __forceinline__ void copy_rows_of_head(const PrologueArgs& a, int h) {
-  constexpr int kTpr = D / 8;
-  constexpr int kRpp = kThreads / kTpr;
-  const int b = blockIdx.z;
-  const int row0 = blockIdx.y * a.group * a.bs;
-  const int rows = min(a.group * a.bs, a.S - row0);
-  const int cg = threadIdx.x % kTpr, rg = threadIdx.x / kTpr;
-  const T* src = static_cast<const T*>(a.in[2]) + (static_cast<int64_t>(b) * a.S + row0) * a.token_stride + h * D + cg * 8;
-  T* dst = static_cast<T*>(a.out[2]) + ((static_cast<int64_t>(b) * a.H + h) * a.N_out + a.dst_row0 + row0) * D + cg * 8;
-  for (int base = rg; base < rows; base += 8 * kRpp) {
-    uint4 v[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int r = base + u * kRpp;
-      if (r < rows) v[u] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<int64_t>(r) * a.token_stride));
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int r = base + u * kRpp;
-      if (r < rows) *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(r) * D) = v[u];
-    }
-  }
-}
-
 template <typename T, int D, int kNorm, int kRope>
-__global__ void __launch_bounds__(kThreads, 2) qkv_prologue_kernel(const __grid_constant__ PrologueArgs a) {
+__global__ void __launch_bounds__(kThreads, 4) qkv_prologue_kernel(const __grid_constant__ PrologueArgs a) {
   constexpr int kTpr = D / 8;               // threads per row
   constexpr int kRpp = kThreads / kTpr;     // rows per pass
   constexpr float kInvD = 1.0f / D;         // D is a power of two: the product equals the division
@@ -136,77 +103,52 @@ __global__ void __launch_bounds__(kThreads, 2) qkv_prologue_kernel(const __grid_
   constexpr int kTabC = kRope == MODDIT_ROPE_PAIR ? 4 : 8;          // table values per thread and row
   __shared__ float red[kRpp][D];
 
-  const int head_groups = (a.H + kHeads - 1) / kHeads;
-  if (static_cast<int>(blockIdx.x) >= head_groups) {
-    if (a.in[2] != nullptr) copy_rows_of_head<T, D>(a, static_cast<int>(blockIdx.x) - head_groups);
-    return;
-  }
-  if (a.in[0] == nullptr && a.in[1] == nullptr) return;
-  const int h0 = blockIdx.x * kHeads;
+  const int which = blockIdx.x / a.H;
+  const int h = blockIdx.x - which * a.H;
   const int b = blockIdx.z;
+  const T* __restrict__ in = static_cast<const T*>(a.in[which]);
+  if (in == nullptr) return;
+  T* __restrict__ out = static_cast<T*>(a.out[which]);
   const int blk0 = blockIdx.y * a.group;    // first token block of this CTA
   const int row0 = blk0 * a.bs;
   const int rows = min(a.group * a.bs, a.S - row0);
   const int spb = a.group > 1 ? a.bs / kRpp : 0;   // load slots per block when the CTA holds several blocks
   const int cg = threadIdx.x % kTpr;
   const int rg = threadIdx.x / kTpr;
-  const bool rope_on = a.cos != nullptr;
-  // the same for the whole CTA
-  auto present = [&](int c) -> bool { return a.in[c & 1] != nullptr && h0 + c / 2 < a.H; };
-  const bool pooled = a.pool[0] != nullptr || a.pool[1] != nullptr;
+  const bool normed = kNorm != MODDIT_NORM_NONE && which < 2;
+  const bool rope_on = which < 2 && a.cos != nullptr;
+  float* pool = which < 2 ? a.pool[which] : nullptr;
 
-  // weight (and bias) of this thread's eight columns: one per tensor, or one per unit when the weight spans the heads
-  constexpr int kWeights = kNorm == MODDIT_NORM_NONE ? 1 : kNorm == MODDIT_NORM_RMS_ALL_HEADS ? kUnits : 2;
-  constexpr int kBiases = kNorm == MODDIT_NORM_LAYER ? 2 : 1;
-  uint4 w2[kWeights], b2[kBiases];
-#pragma unroll
-  for (int c = 0; c < kWeights; ++c) {
-    w2[c] = make_uint4(0, 0, 0, 0);
-    if (kNorm != MODDIT_NORM_NONE && present(c) && a.weight[c & 1] != nullptr) {
-      const int wofs = (kNorm == MODDIT_NORM_RMS_ALL_HEADS ? (h0 + c / 2) * D : 0) + cg * 8;
-      w2[c] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.weight[c & 1]) + wofs));
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < kBiases; ++c) {
-    b2[c] = make_uint4(0, 0, 0, 0);
-    if (kNorm == MODDIT_NORM_LAYER && a.bias[c & 1] != nullptr)
-      b2[c] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.bias[c & 1]) + cg * 8));
+  // weight (and bias) of this thread's eight columns
+  uint4 w2 = make_uint4(0, 0, 0, 0), b2 = make_uint4(0, 0, 0, 0);
+  bool has_w = false;
+  if (normed) {
+    const int wofs = (kNorm == MODDIT_NORM_RMS_ALL_HEADS ? h * D : 0) + cg * 8;
+    has_w = a.weight[which] != nullptr;
+    if (has_w) w2 = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.weight[which]) + wofs));
+    if (kNorm == MODDIT_NORM_LAYER && a.bias[which] != nullptr)
+      b2 = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.bias[which]) + wofs));
   }
 
-  // offsets of row 0 of this CTA at head h0; a unit's head adds D to the source, N_out * D to the destination
-  const int64_t src0 = (static_cast<int64_t>(b) * a.S + row0) * a.token_stride + h0 * D + cg * 8;
-  const int64_t dst0 = ((static_cast<int64_t>(b) * a.H + h0) * a.N_out + a.dst_row0 + row0) * D + cg * 8;
-  const int64_t dst_head = static_cast<int64_t>(a.N_out) * D;
+  const T* src = in + (static_cast<int64_t>(b) * a.S + row0) * a.token_stride + h * D + cg * 8;
+  T* dst = out + ((static_cast<int64_t>(b) * a.H + h) * a.N_out + a.dst_row0 + row0) * D + cg * 8;
   // table entries of row r of this CTA start at tab + r * kTabW (32-bit offsets: the host checks the size)
   const int tab = (row0 - a.rope_lo) * kTabW + cg * kTabC;
 
-  float acc[kUnits][8];
-#pragma unroll
-  for (int c = 0; c < kUnits; ++c)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[c][i] = 0.f;
-  // Means of block blk0 + j from the threads' partial sums, in the order pool_blocks_kernel adds them.
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  // Mean of block blk0 + j from the threads' partial sums, in the order pool_blocks_kernel adds them.
   auto flush = [&](int j, int block_rows) {
 #pragma unroll
-    for (int c = 0; c < kUnits; ++c) {
-      float* pool = a.pool[c & 1];
-      if (!present(c) || pool == nullptr) continue;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        red[rg][cg * 8 + i] = acc[c][i];
-        acc[c][i] = 0.f;
-      }
-      __syncthreads();
-      if (threadIdx.x < D) {
-        float t = 0.f;
+    for (int i = 0; i < 8; ++i) red[rg][cg * 8 + i] = acc[i];
+    __syncthreads();
+    if (threadIdx.x < D) {
+      float t = 0.f;
 #pragma unroll 8
-        for (int g = 0; g < kRpp; ++g) t += red[g][threadIdx.x];
-        pool[((static_cast<int64_t>(b) * a.H + h0 + c / 2) * a.nb_total + a.blk_base + blk0 + j) * D + threadIdx.x] =
-            t / static_cast<float>(block_rows);
-      }
-      __syncthreads();
+      for (int g = 0; g < kRpp; ++g) t += red[g][threadIdx.x];
+      pool[((static_cast<int64_t>(b) * a.H + h) * a.nb_total + a.blk_base + blk0 + j) * D + threadIdx.x] =
+          t / static_cast<float>(block_rows);
     }
+    __syncthreads();
   };
 
   // kWhole: the CTA has all of its 8 * kRpp rows and they are rotated all or none - no test per row.
@@ -214,26 +156,20 @@ __global__ void __launch_bounds__(kThreads, 2) qkv_prologue_kernel(const __grid_
     constexpr bool kWhole = decltype(whole_tag)::value;
     const bool rope_all = rope_on && row0 >= a.rope_lo && row0 < a.rope_hi;      // only read when kWhole
     for (int base = 0; base < rows; base += 8 * kRpp) {     // uniform trip count: the shuffles need every lane
-      auto fetch = [&](uint4 (&v)[kUnits], int r) {
-        const bool valid = kWhole || r < rows;
+      uint4 v[8];
 #pragma unroll
-        for (int c = 0; c < kUnits; ++c)
-          v[c] = (valid && present(c))
-                     ? __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(a.in[c & 1]) + src0 + (c / 2) * D +
-                                                            static_cast<int64_t>(r) * a.token_stride))
-                     : make_uint4(0, 0, 0, 0);
-      };
-      auto rotated = [&](int r) -> bool {
-        return kWhole ? rope_all : (rope_on && r < rows && row0 + r >= a.rope_lo && row0 + r < a.rope_hi);
-      };
-      uint4 next[kUnits];
-      fetch(next, base + rg);
+      for (int u = 0; u < 8; ++u) {
+        const int r = base + rg + u * kRpp;
+        v[u] = (kWhole || r < rows) ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<int64_t>(r) * a.token_stride))
+                                    : make_uint4(0, 0, 0, 0);
+      }
       if (rope_on) {
         // the table rows are needed one after the other below: ask for all of them now
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int r = base + rg + u * kRpp;
-          if (rotated(r)) {
+          const int s = row0 + r;
+          if (kWhole ? rope_all : (r < rows && s >= a.rope_lo && s < a.rope_hi)) {
             asm volatile("prefetch.global.L1 [%0];" ::"l"(a.cos + tab + r * kTabW));
             asm volatile("prefetch.global.L1 [%0];" ::"l"(a.sin + tab + r * kTabW));
           }
@@ -244,25 +180,8 @@ __global__ void __launch_bounds__(kThreads, 2) qkv_prologue_kernel(const __grid_
         const int r = base + rg + u * kRpp;
         const bool valid = kWhole || r < rows;
         const int s = row0 + r;               // token index within the input
-        uint4 v[kUnits];
-#pragma unroll
-        for (int c = 0; c < kUnits; ++c) v[c] = next[c];
-        if (u + 1 < 8) fetch(next, r + kRpp);  // the next row's four pieces travel while this row is worked on
-        const bool rope = rotated(r);
-        float cs[kTabC], sn[kTabC];
-        if (rope) {
-#pragma unroll
-          for (int i = 0; i < kTabC; i += 4) {
-            *reinterpret_cast<float4*>(cs + i) = __ldg(reinterpret_cast<const float4*>(a.cos + tab + r * kTabW + i));
-            *reinterpret_cast<float4*>(sn + i) = __ldg(reinterpret_cast<const float4*>(a.sin + tab + r * kTabW + i));
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < kUnits; ++c) {
-          if (!present(c)) continue;
-          const uint4 wv2 = w2[kWeights == 1 ? 0 : c % kWeights];
-          const bool has_w = kNorm != MODDIT_NORM_NONE && a.weight[c & 1] != nullptr;
-          uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+        uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+        if (normed) {
           if constexpr (kNorm == MODDIT_NORM_RMS_HEAD || kNorm == MODDIT_NORM_RMS_ALL_HEADS) {
             float rs;
             if constexpr (kNorm == MODDIT_NORM_RMS_HEAD) {
@@ -275,10 +194,10 @@ __global__ void __launch_bounds__(kThreads, 2) qkv_prologue_kernel(const __grid_
               }
               rs = rsqrtf(__fadd_rn(row_sum<kTpr>(ss) * kInvD, a.eps));
             } else {
-              rs = valid ? __ldg(a.inv_rms[c & 1] + static_cast<int64_t>(b) * a.S + s) : 0.f;
+              rs = valid ? __ldg(a.inv_rms[which] + static_cast<int64_t>(b) * a.S + s) : 0.f;
             }
             // x * rsqrt in float32 rounded to T, then the product with the weight rounded to T again
-            const uint32_t wt[4] = {wv2.x, wv2.y, wv2.z, wv2.w};
+            const uint32_t wt[4] = {w2.x, w2.y, w2.z, w2.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               w[i] = Pair<T>::pack(__fmul_rn(Pair<T>::lo(w[i]), rs), __fmul_rn(Pair<T>::hi(w[i]), rs));
@@ -286,9 +205,9 @@ __global__ void __launch_bounds__(kThreads, 2) qkv_prologue_kernel(const __grid_
             }
           } else if constexpr (kNorm == MODDIT_NORM_LAYER) {
             float f[8], wv[8], bv[8];
-            unpack<T>(v[c], f);
-            unpack<T>(wv2, wv);
-            unpack<T>(b2[c % kBiases], bv);
+            unpack<T>(v[u], f);
+            unpack<T>(w2, wv);
+            unpack<T>(b2, bv);
             float sum = 0.f;
 #pragma unroll
             for (int i = 0; i < 8; ++i) sum += f[i];
@@ -307,32 +226,42 @@ __global__ void __launch_bounds__(kThreads, 2) qkv_prologue_kernel(const __grid_
               w[i] = valid ? Pair<T>::pack(y0, y1) : 0u;
             }
           }
-          if (rope) {
+        }
+        if (kWhole ? rope_all : (rope_on && valid && s >= a.rope_lo && s < a.rope_hi)) {
+          float c[kTabC], n[kTabC];
+          const float* cp = a.cos + tab + r * kTabW;
+          const float* np = a.sin + tab + r * kTabW;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              // multipliers of (x0, x1) for the even element (ce, se) and for the odd element (so, co)
-              const float ce = kRope == MODDIT_ROPE_PAIR ? cs[i] : cs[2 * i];
-              const float co = kRope == MODDIT_ROPE_PAIR ? cs[i] : (kRope == MODDIT_ROPE_ELEMENTWISE ? cs[2 * i + 1] : cs[2 * i]);
-              const float se = kRope == MODDIT_ROPE_PAIR ? sn[i] : (kRope == MODDIT_ROPE_ELEMENTWISE ? sn[2 * i] : sn[2 * i + 1]);
-              const float so = kRope == MODDIT_ROPE_PAIR ? sn[i] : sn[2 * i + 1];
-              const float x0 = Pair<T>::lo(w[i]), x1 = Pair<T>::hi(w[i]);
-              // products rounded separately, then one add (no fused multiply-add), as a tensor expression does
-              w[i] = Pair<T>::pack(__fsub_rn(__fmul_rn(x0, ce), __fmul_rn(x1, se)),
-                                   __fadd_rn(__fmul_rn(x0, so), __fmul_rn(x1, co)));
-            }
+          for (int i = 0; i < kTabC; i += 4) {
+            *reinterpret_cast<float4*>(c + i) = __ldg(reinterpret_cast<const float4*>(cp + i));
+            *reinterpret_cast<float4*>(n + i) = __ldg(reinterpret_cast<const float4*>(np + i));
           }
-          if (valid)
-            *reinterpret_cast<uint4*>(static_cast<T*>(a.out[c & 1]) + dst0 + (c / 2) * dst_head + static_cast<int64_t>(r) * D) =
-                make_uint4(w[0], w[1], w[2], w[3]);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {        // rows past the end hold zeros here
-            acc[c][2 * i] += Pair<T>::lo(w[i]);
-            acc[c][2 * i + 1] += Pair<T>::hi(w[i]);
+          for (int i = 0; i < 4; ++i) {
+            // multipliers of (x0, x1) for the even element (ce, se) and for the odd element (so, co)
+            const float ce = kRope == MODDIT_ROPE_PAIR ? c[i] : c[2 * i];
+            const float co = kRope == MODDIT_ROPE_PAIR ? c[i] : (kRope == MODDIT_ROPE_ELEMENTWISE ? c[2 * i + 1] : c[2 * i]);
+            const float se = kRope == MODDIT_ROPE_PAIR ? n[i] : (kRope == MODDIT_ROPE_ELEMENTWISE ? n[2 * i] : n[2 * i + 1]);
+            const float so = kRope == MODDIT_ROPE_PAIR ? n[i] : n[2 * i + 1];
+            const float x0 = Pair<T>::lo(w[i]), x1 = Pair<T>::hi(w[i]);
+            // products rounded separately, then one add (no fused multiply-add), as a tensor expression does
+            w[i] = Pair<T>::pack(__fsub_rn(__fmul_rn(x0, ce), __fmul_rn(x1, se)),
+                                 __fadd_rn(__fmul_rn(x0, so), __fmul_rn(x1, co)));
           }
         }
-        if (pooled && spb > 0 && (u + 1) % spb == 0) {   // last slot of a block (the same for every thread)
-          const int j = u / spb;
-          if (j * a.bs < rows) flush(j, min(a.bs, rows - j * a.bs));
+        if (valid) *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(r) * D) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (pool != nullptr) {                 // rows past the end hold zeros here
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            acc[2 * i] += Pair<T>::lo(w[i]);
+            acc[2 * i + 1] += Pair<T>::hi(w[i]);
+          }
+          if (spb > 0 && (u + 1) % spb == 0) {  // last slot of a block (the same for every thread)
+            const int j = u / spb;
+            if (j * a.bs < rows) flush(j, min(a.bs, rows - j * a.bs));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+          }
         }
       }
     }
@@ -343,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 2) qkv_prologue_kernel(const __grid_
     run(std::true_type{});
   else
     run(std::false_type{});
-  if (pooled && spb == 0) flush(0, rows);
+  if (pool != nullptr && spb == 0) flush(0, rows);
 }
 
 // One warp per token: 1/sqrt(mean of squares over the whole H*D row + eps) for the normalisation that spans
@@ -382,7 +311,7 @@ int launch_prologue(const PrologueArgs& a, int B, int D, int norm_kind, int64_t 
                                                        tokens, token_stride, a.H * D, a.eps, ws, ws + tokens);
     MODDIT_CHECK_LAUNCH("token_inv_rms_kernel");
   }
-  const dim3 grid(ceil_div(a.H, kHeads) + a.H, ceil_div(a.S, a.bs * a.group), B);
+  const dim3 grid(3 * a.H, ceil_div(a.S, a.bs * a.group), B);
 #define MODDIT_PROLOGUE_ROPE(NORM, ROPE)                                        \
   case ROPE:                                                                    \
     if (D == 64)                                                                \
