@@ -71,11 +71,12 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 
 // ---- long lists in parts -----------------------------------------------------------------------------------------
 // The pairs of text rows keep every key tile, several times the average list.  In a launch of a few hundred items such a
-// list is the launch's end: 8,448 tokens, four heads: 66 entries against 24 on average, 122 us of which the last half
-// runs on eight SMs.  So the (at most) two longest lists of a head, if they exceed 3/2 of its mean, are walked by up to
-// kMaxParts CTAs of about a mean list each; every part leaves its unnormalised rows with their maximum and sum in a
-// workspace, and a second small kernel puts the parts together.  The rule looks at one head's lists only, so a row's
-// result does not depend on what else is in the launch.  Past kSplitPairs pairs a head has enough items of its own.
+// list is the launch's end: 8,448 tokens, four heads, 66 entries against 24 on average: 127 us, in parts 81 us with the
+// kernel that puts them together.  So the (at most) two longest lists of a head, if they exceed 3/2 of its mean, are
+// walked by up to kMaxParts CTAs of about a mean list each; every part leaves its unnormalised rows with their maximum
+// and sum in a workspace, and a second small kernel puts the parts together.  The rule looks at one head's lists only,
+// so a row's result does not depend on what else is in the launch.  Past kSplitPairs pairs a head has enough items of
+// its own and the look at the lists costs more than it gives (16,640 tokens, 32 heads: 1235 us, in parts 1263).
 constexpr int kLongPairs = 2;        // the pairs that the start order puts first
 constexpr int kMaxParts = 4;
 constexpr int kSplitPairs = 64;      // 16,384 tokens
