@@ -317,20 +317,6 @@ int moddit_sparse_attn_fwd(const void* q, const void* k, const void* v, int dtyp
                            float softmax_scale, int q_split, int kv_len_lo, int kv_len_hi, void* out,
                            float* lse, int32_t* status, void* stream);
 
-/* The same forward with the one or two longest lists of a mask head walked in up to four parts by as many blocks, where
- * they are more than 3/2 of that head's mean list (text rows beside sparse video rows): in a launch of a few hundred
- * items such a list is what the launch waits for at its end.  The parts' float32 rows go through the workspace
- * (moddit_sparse_attn_fwd_split_bytes(...) bytes, 16-byte aligned; 0 for sequences past 16,384 tokens, which are never
- * divided) and a second kernel puts them together, so rows of divided lists differ from moddit_sparse_attn_fwd in
- * rounding.  n_peers = 0: rows to `out`; n_peers > 0: rows to the peers as moddit_sparse_attn_fwd_scatter stores them.
- */
-size_t moddit_sparse_attn_fwd_split_bytes(int BH, int N, int D);
-int moddit_sparse_attn_fwd_split(const void* q, const void* k, const void* v, int dtype, int BH, int N, int D,
-                                 const int32_t* counts, const int32_t* entries, const int32_t* order, int Hm,
-                                 float softmax_scale, int q_split, int kv_len_lo, int kv_len_hi, void* out,
-                                 void* const* peer_out, int n_peers, int head_base, float* lse, int32_t* status,
-                                 void* workspace, size_t workspace_bytes, void* stream);
-
 /* ---------------------------------------------------------------------------------------------
  * Strided row copy: `rows` rows of `width_bytes` bytes from src (pitch src_pitch) to dst (pitch dst_pitch).
  * `dst` may be a peer GPU's memory mapped into this process; the kernel uses plain loads and stores.  It is

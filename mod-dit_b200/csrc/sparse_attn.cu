@@ -58,189 +58,6 @@ struct OutScatter {
   int head_base;
 };
 
-template <bool kBF16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (kBF16) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  } else {
-    const __half2 v = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  }
-}
-
-// ---- long lists in parts -----------------------------------------------------------------------------------------
-// The pairs of text rows keep every key tile, several times the average list.  In a launch of a few hundred items such a
-// list is the launch's end: 8,448 tokens, four heads, 66 entries against 24 on average: 127 us, in parts 81 us with the
-// kernel that puts them together.  So the (at most) two longest lists of a head, if they exceed 3/2 of its mean, are
-// walked by up to kMaxParts CTAs of about a mean list each; every part leaves its unnormalised rows with their maximum
-// and sum in a workspace, and a second small kernel puts the parts together.  The rule looks at one head's lists only,
-// so a row's result does not depend on what else is in the launch.  Past kSplitPairs pairs a head has enough items of
-// its own and the look at the lists costs more than it gives (16,640 tokens, 32 heads: 1235 us, in parts 1263).
-constexpr int kLongPairs = 2;        // the pairs that the start order puts first
-constexpr int kMaxParts = 4;
-constexpr int kSplitPairs = 64;      // 16,384 tokens
-constexpr int kExtra = kLongPairs * (kMaxParts - 1);      // CTAs per head for parts 1, 2, ...
-
-struct SplitArgs {
-  float* partial;       // (BH, kLongPairs, kMaxParts, 256, D + 2) float32, or NULL: every list in one piece
-  int npairs;
-};
-
-struct LongPair { int pair, count, parts; };     // parts == 1: not divided
-
-// The head's longest (rank 0) and second longest list (ties by index), and in how many parts they are walked.
-// Whole warps; npairs <= kSplitPairs.
-__device__ __forceinline__ void long_pairs(const int32_t* __restrict__ counts, int npairs, int lane, LongPair (&lp)[kLongPairs]) {
-  unsigned key[kSplitPairs / 32];
-  unsigned sum = 0;
-#pragma unroll
-  for (int u = 0; u < kSplitPairs / 32; ++u) {
-    const int i = lane + 32 * u;
-    const unsigned c = i < npairs ? static_cast<unsigned>(counts[i]) : 0u;
-    sum += c;
-    key[u] = i < npairs ? ((c + 1u) << 9) | static_cast<unsigned>(511 - i) : 0u;      // lists have at most 128 entries
-  }
-  const unsigned total = __reduce_add_sync(0xffffffffu, sum);
-  const int mean = max(1, static_cast<int>((total + npairs - 1) / npairs));
-  unsigned taken = 0xffffffffu;
-#pragma unroll
-  for (int r = 0; r < kLongPairs; ++r) {
-    unsigned best = 0;
-#pragma unroll
-    for (int u = 0; u < kSplitPairs / 32; ++u) best = max(best, key[u] < taken ? key[u] : 0u);
-    best = __reduce_max_sync(0xffffffffu, best);
-    taken = best;
-    lp[r].pair = best ? 511 - static_cast<int>(best & 511u) : -1;
-    lp[r].count = best ? static_cast<int>(best >> 9) - 1 : 0;
-    lp[r].parts = 2 * lp[r].count > 3 * mean ? min(kMaxParts, (lp[r].count + mean - 1) / mean) : 1;
-  }
-}
-
-// What a CTA walks: the whole list of its item, or part `part` of `parts` of it.
-struct WorkItem { int mh, pair, begin, end, rank, part, parts; };
-
-// false: nothing to do (a part that this head does not have)
-__device__ __forceinline__ bool find_work(const int32_t* __restrict__ counts, const int32_t* __restrict__ order, int Hm,
-                                          const SplitArgs& split, int lane, WorkItem& w) {
-  const int npairs = split.npairs;
-  const int extra = split.partial != nullptr ? kExtra * Hm : 0;
-  w.rank = -1;
-  w.part = 0;
-  w.parts = 1;
-  const int x = static_cast<int>(blockIdx.x);
-  if (x >= extra) {
-    const int item = order ? order[x - extra] : x - extra;
-    w.mh = item / npairs;
-    w.pair = item - w.mh * npairs;
-  } else {
-    w.mh = x / kExtra;
-  }
-  const int32_t* c = counts + static_cast<int64_t>(w.mh) * npairs;
-  if (split.partial != nullptr) {
-    LongPair lp[kLongPairs];
-    long_pairs(c, npairs, lane, lp);
-    if (x < extra) {
-      w.rank = (x - w.mh * kExtra) / (kMaxParts - 1);
-      w.part = 1 + (x - w.mh * kExtra) % (kMaxParts - 1);
-      w.pair = w.rank == 0 ? lp[0].pair : lp[1].pair;
-    } else {
-      w.rank = w.pair == lp[0].pair ? 0 : w.pair == lp[1].pair ? 1 : -1;
-    }
-    if (w.rank >= 0) w.parts = w.rank == 0 ? lp[0].parts : lp[1].parts;
-    if (w.part >= w.parts && x < extra) return false;
-  }
-  const int cnt = c[w.pair];
-  const int len = (cnt + w.parts - 1) / w.parts;
-  w.begin = min(cnt, w.part * len);
-  w.end = min(cnt, w.begin + len);
-  return true;
-}
-
-// Rows of one part: D unnormalised sums, then the row's reference (log2 domain) and its sum.
-template <int D>
-__device__ __forceinline__ float* partial_row(float* partial, int bh, int rank, int part, int row) {
-  return partial + (((static_cast<int64_t>(bh) * kLongPairs + rank) * kMaxParts + part) * 256 + row) * (D + 2);
-}
-
-template <int D>
-__device__ __forceinline__ void store_partial(float* dst, uint32_t tO, bool any, float m, float l) {
-#pragma unroll
-  for (int c = 0; c < D / 32; ++c) {
-    float o[32];
-    if (any) {
-      ptx::tmem_ld32(tO + c * 32, reinterpret_cast<uint32_t*>(o));
-      ptx::tmem_ld_wait();
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) o[i] = 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) *reinterpret_cast<float2*>(dst + c * 32 + i) = make_float2(o[i], o[i + 1]);
-  }
-  *reinterpret_cast<float2*>(dst + D) = make_float2(m, l);
-}
-
-// Puts the parts of the divided lists together.  Grid: x = 16 rows, y = long pair of a mask head, z = batch; a warp per
-// row, two rows one after the other.
-template <int D, bool kBF16>
-__global__ void __launch_bounds__(256) combine_parts_kernel(const int32_t* __restrict__ counts, int Hm, int N,
-                                                            const __grid_constant__ SplitArgs split, void* __restrict__ out_raw,
-                                                            float* __restrict__ lse, const __grid_constant__ OutScatter scatter) {
-  const int lane = threadIdx.x % 32;
-  const int mh = blockIdx.y / kLongPairs, rank = blockIdx.y % kLongPairs;
-  LongPair lp[kLongPairs];
-  long_pairs(counts + static_cast<int64_t>(mh) * split.npairs, split.npairs, lane, lp);
-  const int pair = rank == 0 ? lp[0].pair : lp[1].pair, parts = rank == 0 ? lp[0].parts : lp[1].parts;
-  if (parts < 2) return;
-  const int bh = blockIdx.z * Hm + mh;
-  constexpr int kPer = D / 32;           // consecutive columns per lane
-  for (int r = blockIdx.x * 16 + threadIdx.x / 32; r < blockIdx.x * 16 + 16; r += 8) {
-    const int grow = pair * 256 + r;
-    if (grow >= N) continue;
-    float o[kMaxParts][kPer], m[kMaxParts], l[kMaxParts];
-    float M = -INFINITY;
-#pragma unroll
-    for (int t = 0; t < kMaxParts; ++t) {
-      m[t] = -INFINITY;
-      l[t] = 0.f;
-      if (t < parts) {
-        const float* src = partial_row<D>(split.partial, bh, rank, t, r);
-#pragma unroll
-        for (int i = 0; i < kPer; i += 2) *reinterpret_cast<float2*>(&o[t][i]) = *reinterpret_cast<const float2*>(src + lane * kPer + i);
-        const float2 ml = *reinterpret_cast<const float2*>(src + D);
-        m[t] = ml.x;
-        l[t] = ml.y;
-      }
-      M = fmaxf(M, m[t]);
-    }
-    const float ref = (M == -INFINITY) ? 0.f : M;
-    float acc[kPer] = {}, L = 0.f;
-#pragma unroll
-    for (int t = 0; t < kMaxParts; ++t) {
-      if (t >= parts) continue;
-      const float f = exp2f(m[t] - ref);           // a part without a key: 2^-inf = 0 times its zeros
-      L = fmaf(l[t], f, L);
-#pragma unroll
-      for (int i = 0; i < kPer; ++i) acc[i] = fmaf(o[t][i], f, acc[i]);
-    }
-    const float inv = L > 0.f ? 1.f / L : (L == 0.f ? 0.f : L);     // no key at all: zeros; NaN stays NaN
-    unsigned char* dst;
-    if (scatter.n_peers > 0) {
-      const int pr = min(grow / scatter.rows_per_peer, scatter.n_peers - 1);
-      dst = static_cast<unsigned char*>(scatter.peer[pr]) +
-            (static_cast<int64_t>(scatter.head_base + bh) * scatter.rows_per_peer + (grow - pr * scatter.rows_per_peer)) * D * 2;
-    } else {
-      dst = static_cast<unsigned char*>(out_raw) + (static_cast<int64_t>(bh) * N + grow) * D * 2;
-    }
-    uint32_t* dst32 = reinterpret_cast<uint32_t*>(dst) + lane * (kPer / 2);
-#pragma unroll
-    for (int i = 0; i < kPer; i += 2) dst32[i / 2] = pack2<kBF16>(acc[i] * inv, acc[i + 1] * inv);
-    if (lse != nullptr && lane == 0)
-      lse[static_cast<int64_t>(bh) * N + grow] = L > 0.f ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
-  }
-}
-
 struct __align__(8) Control {
   unsigned long long bars[kNumBarriers];
   uint32_t tmem_base;
@@ -261,13 +78,24 @@ __device__ __forceinline__ void report(int32_t* status, int code, int role, int 
   }
 }
 
+template <bool kBF16>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  if constexpr (kBF16) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+
 template <int D, bool kBF16>
 __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
     const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
     const __grid_constant__ CUtensorMap tm_v, const int32_t* __restrict__ counts,
     const int32_t* __restrict__ entries, const int32_t* __restrict__ order, int Hm, int ntk, int N, float scale_log2, int q_split, int kvl_lo,
     int kvl_hi, void* __restrict__ out_raw, float* __restrict__ lse, int32_t* __restrict__ status,
-    const __grid_constant__ OutScatter scatter, const __grid_constant__ SplitArgs split) {
+    const __grid_constant__ OutScatter scatter) {
   constexpr int kTileBytes = kTile * D * 2;       // one Q, K or V tile
   constexpr int kChunks = D / 64;                 // 64-element (128-byte) column chunks per tile
   constexpr int kChunkBytes = kTile * 128;
@@ -286,19 +114,17 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
 
   const int warp = ptx::warp_index();
   const int lane = threadIdx.x % 32;
-  // grid: x = parts 1, 2, ... of divided lists, then work items (mask head, query-tile pair); y = batch.  Blocks start
-  // in increasing blockIdx.x; `order` (from the work-list builder) puts long lists first, otherwise items run head by
-  // head.
-  WorkItem work;
-  if (!find_work(counts, order, Hm, split, lane, work)) return;
-  const int npairs = split.npairs;
-  const int mh = work.mh;
-  const int pair = work.pair;
+  // grid: x = work item (mask head, query-tile pair), y = batch.  Blocks start in increasing blockIdx.x;
+  // `order` (from the work-list builder) puts long lists first, otherwise items run head by head.
+  const int npairs = static_cast<int>(gridDim.x) / Hm;
+  const int item = order ? order[blockIdx.x] : static_cast<int>(blockIdx.x);
+  const int mh = item / npairs;
+  const int pair = item - mh * npairs;
   const int bh = blockIdx.y * Hm + mh;
   const int ntq = (N + kTile - 1) / kTile;
   const bool has_b = (2 * pair + 1) < ntq;
-  const int cnt = work.end - work.begin;
-  const int32_t* ent = entries + (static_cast<int64_t>(mh) * npairs + pair) * ntk + work.begin;
+  const int cnt = counts[static_cast<int64_t>(mh) * npairs + pair];
+  const int32_t* ent = entries + (static_cast<int64_t>(mh) * npairs + pair) * ntk;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kNumBarriers; ++i) ptx::mbar_init(bar(i), (i >= kPLoA && i <= kPHiB) ? 128u : 1u);
@@ -576,10 +402,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
       ok = __all_sync(0xffffffffu, ok);
       if (!ok && lane == 0) report(status, 5, 2 + x, -1);
     }
-    if (ok && tile < ntq && work.parts > 1) {
-      ptx::tc_fence_after();
-      store_partial<D>(partial_row<D>(split.partial, bh, work.rank, work.part, x * kTile + r), tO, done > 0, m, l);
-    } else if (ok && tile < ntq) {
+    if (ok && tile < ntq) {
       ptx::tc_fence_after();
       const float inv = (done > 0 && l > 0.f) ? 1.f / l : 0.f;
       uint4* dst;
@@ -750,8 +573,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
     const __grid_constant__ CUtensorMap tm_v, const int32_t* __restrict__ counts,
     const int32_t* __restrict__ entries, const int32_t* __restrict__ order, int Hm, int ntk, int N, float scale_log2,
     int q_split, int kvl_lo, int kvl_hi, void* __restrict__ out_raw, float* __restrict__ lse,
-    int32_t* __restrict__ status, const __grid_constant__ OutScatter scatter,
-    const __grid_constant__ SplitArgs split) {
+    int32_t* __restrict__ status, const __grid_constant__ OutScatter scatter) {
   constexpr int D = 64;
   constexpr int kTileBytes = kTile * D * 2;       // one Q, K or V tile: 128 rows x 128 bytes
   constexpr uint32_t kIdescQK = ptx::idesc_f16(128, 128, kBF16, false);
@@ -769,16 +591,15 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
 
   const int warp = ptx::warp_index();
   const int lane = threadIdx.x % 32;
-  WorkItem work;
-  if (!find_work(counts, order, Hm, split, lane, work)) return;
-  const int npairs = split.npairs;
-  const int mh = work.mh;
-  const int pair = work.pair;
+  const int npairs = static_cast<int>(gridDim.x) / Hm;
+  const int item = order ? order[blockIdx.x] : static_cast<int>(blockIdx.x);
+  const int mh = item / npairs;
+  const int pair = item - mh * npairs;
   const int bh = blockIdx.y * Hm + mh;
   const int ntq = (N + kTile - 1) / kTile;
   const bool has_b = (2 * pair + 1) < ntq;
-  const int cnt = work.end - work.begin;
-  const int32_t* ent = entries + (static_cast<int64_t>(mh) * npairs + pair) * ntk + work.begin;
+  const int cnt = counts[static_cast<int64_t>(mh) * npairs + pair];
+  const int32_t* ent = entries + (static_cast<int64_t>(mh) * npairs + pair) * ntk;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < k6NumBarriers; ++i) {
@@ -1032,10 +853,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
       ok = __all_sync(0xffffffffu, ok);
       if (!ok && lane == 0) report(status, 5, 2 + x, -1);
     }
-    if (ok && tile < ntq && work.parts > 1) {
-      ptx::tc_fence_after();
-      store_partial<D>(partial_row<D>(split.partial, bh, work.rank, work.part, x * kTile + r), tO, done > 0, m, l);
-    } else if (ok && tile < ntq) {
+    if (ok && tile < ntq) {
       ptx::tc_fence_after();
       const float inv = (done > 0 && l > 0.f) ? 1.f / l : 0.f;
       uint4* dst;
@@ -1087,8 +905,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
 template <bool kBF16>
 int launch_d64(const void* q, const void* k, const void* v, int dtype, int BH, int N, const int32_t* counts,
                const int32_t* entries, const int32_t* order, int Hm, float softmax_scale, int q_split, int kvl_lo,
-               int kvl_hi, void* out, float* lse, int32_t* status, const OutScatter& scatter, float* partial,
-               cudaStream_t st) {
+               int kvl_hi, void* out, float* lse, int32_t* status, const OutScatter& scatter, cudaStream_t st) {
   CUtensorMap tq, tk, tv;
   if (int rc = make_tmap_rows(&tq, q, dtype, BH, N, 64, kTile)) return rc;
   if (int rc = make_tmap_rows(&tk, k, dtype, BH, N, 64, kTile)) return rc;
@@ -1099,23 +916,16 @@ int launch_d64(const void* q, const void* k, const void* v, int dtype, int BH, i
   const size_t smem = smem_bytes_d64();
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  const SplitArgs split = {npairs <= kSplitPairs ? partial : nullptr, npairs};
-  const int extra = split.partial != nullptr ? kExtra * Hm : 0;
-  kernel<<<dim3(npairs * Hm + extra, BH / Hm), kThreads, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N,
-                                                                    scale_log2, q_split, kvl_lo, kvl_hi, out, lse, status,
-                                                                    scatter, split);
+  kernel<<<dim3(npairs * Hm, BH / Hm), kThreads, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N, scale_log2,
+                                                            q_split, kvl_lo, kvl_hi, out, lse, status, scatter);
   MODDIT_CHECK_LAUNCH("sparse_attn_fwd_d64_kernel");
-  if (extra) {
-    combine_parts_kernel<64, kBF16><<<dim3(16, kLongPairs * Hm, BH / Hm), 256, 0, st>>>(counts, Hm, N, split, out, lse, scatter);
-    MODDIT_CHECK_LAUNCH("combine_parts_kernel");
-  }
   return MODDIT_OK;
 }
 
 template <int D, bool kBF16>
 int launch(const void* q, const void* k, const void* v, int dtype, int BH, int N, const int32_t* counts,
            const int32_t* entries, const int32_t* order, int Hm, float softmax_scale, int q_split, int kvl_lo, int kvl_hi, void* out,
-           float* lse, int32_t* status, const OutScatter& scatter, float* partial, cudaStream_t st) {
+           float* lse, int32_t* status, const OutScatter& scatter, cudaStream_t st) {
   CUtensorMap tq, tk, tv;
   if (int rc = make_tmap_rows(&tq, q, dtype, BH, N, D, kTile)) return rc;
   if (int rc = make_tmap_rows(&tk, k, dtype, BH, N, D, kTile)) return rc;
@@ -1126,16 +936,9 @@ int launch(const void* q, const void* k, const void* v, int dtype, int BH, int N
   const size_t smem = smem_bytes<D>();
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  const SplitArgs split = {npairs <= kSplitPairs ? partial : nullptr, npairs};
-  const int extra = split.partial != nullptr ? kExtra * Hm : 0;
-  kernel<<<dim3(npairs * Hm + extra, BH / Hm), kThreads, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N,
-                                                                    scale_log2, q_split, kvl_lo, kvl_hi, out, lse, status,
-                                                                    scatter, split);
+  kernel<<<dim3(npairs * Hm, BH / Hm), kThreads, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N, scale_log2, q_split,
+                                                   kvl_lo, kvl_hi, out, lse, status, scatter);
   MODDIT_CHECK_LAUNCH("sparse_attn_fwd_kernel");
-  if (extra) {
-    combine_parts_kernel<D, kBF16><<<dim3(16, kLongPairs * Hm, BH / Hm), 256, 0, st>>>(counts, Hm, N, split, out, lse, scatter);
-    MODDIT_CHECK_LAUNCH("combine_parts_kernel");
-  }
   return MODDIT_OK;
 }
 
@@ -1147,7 +950,7 @@ using namespace moddit;
 static int sparse_attn_dispatch(const void* q, const void* k, const void* v, int dtype, int BH, int N, int D,
                                 const int32_t* counts, const int32_t* entries, const int32_t* order, int Hm,
                                 float softmax_scale, int q_split, int kv_len_lo, int kv_len_hi, void* out, float* lse,
-                                int32_t* status, const OutScatter& scatter, float* partial, void* stream) {
+                                int32_t* status, const OutScatter& scatter, void* stream) {
   MODDIT_CHECK_ARG(q && k && v && counts && entries && status, "sparse_attn_fwd: null pointer");
   MODDIT_CHECK_ARG(out || scatter.n_peers > 0, "sparse_attn_fwd: no output destination");
   MODDIT_CHECK_ARG(BH > 0 && BH <= 65535 && N > 0 && Hm > 0, "sparse_attn_fwd: BH=%d N=%d Hm=%d out of range", BH, N, Hm);
@@ -1164,20 +967,20 @@ static int sparse_attn_dispatch(const void* q, const void* k, const void* v, int
   if (D == 128) {
     return dtype == MODDIT_BF16
                ? launch<128, true>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                                   kv_len_hi, out, lse, status, scatter, partial, st)
+                                   kv_len_hi, out, lse, status, scatter, st)
                : launch<128, false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                                    kv_len_hi, out, lse, status, scatter, partial, st);
+                                    kv_len_hi, out, lse, status, scatter, st);
   }
 #ifdef MODDIT_D64_SHARED_KERNEL
   return dtype == MODDIT_BF16 ? launch<64, true>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
-                                                 kv_len_lo, kv_len_hi, out, lse, status, scatter, partial, st)
+                                                 kv_len_lo, kv_len_hi, out, lse, status, scatter, st)
                               : launch<64, false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
-                                                  kv_len_lo, kv_len_hi, out, lse, status, scatter, partial, st);
+                                                  kv_len_lo, kv_len_hi, out, lse, status, scatter, st);
 #else
   return dtype == MODDIT_BF16 ? launch_d64<true>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
-                                                 kv_len_lo, kv_len_hi, out, lse, status, scatter, partial, st)
+                                                 kv_len_lo, kv_len_hi, out, lse, status, scatter, st)
                               : launch_d64<false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
-                                                  kv_len_lo, kv_len_hi, out, lse, status, scatter, partial, st);
+                                                  kv_len_lo, kv_len_hi, out, lse, status, scatter, st);
 #endif
 }
 
@@ -1189,24 +992,7 @@ extern "C" int moddit_sparse_attn_fwd(const void* q, const void* k, const void* 
   MODDIT_CHECK_ARG(out, "sparse_attn_fwd: null output pointer");
   OutScatter none = {};
   return sparse_attn_dispatch(q, k, v, dtype, BH, N, D, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                              kv_len_hi, out, lse, status, none, nullptr, stream);
-}
-
-// Destination table of a scattered output; checks it.
-static int make_scatter(OutScatter* sc, void* const* peer_out, int n_peers, int head_base, int N) {
-  MODDIT_CHECK_ARG(peer_out, "sparse_attn_fwd_scatter: null peer table");
-  MODDIT_CHECK_ARG(n_peers >= 1 && n_peers <= kMaxPeers, "sparse_attn_fwd_scatter: n_peers=%d outside [1, %d]", n_peers,
-                   kMaxPeers);
-  MODDIT_CHECK_ARG(N % n_peers == 0, "sparse_attn_fwd_scatter: N=%d does not divide over %d peers", N, n_peers);
-  MODDIT_CHECK_ARG(head_base >= 0, "sparse_attn_fwd_scatter: head_base must be non-negative");
-  for (int i = 0; i < n_peers; ++i) {
-    MODDIT_CHECK_ARG(peer_out[i] && aligned16(peer_out[i]), "sparse_attn_fwd_scatter: peer buffer %d null or unaligned", i);
-    sc->peer[i] = peer_out[i];
-  }
-  sc->n_peers = n_peers;
-  sc->rows_per_peer = N / n_peers;
-  sc->head_base = head_base;
-  return MODDIT_OK;
+                              kv_len_hi, out, lse, status, none, stream);
 }
 
 extern "C" int moddit_sparse_attn_fwd_scatter(const void* q, const void* k, const void* v, int dtype, int BH, int N,
@@ -1215,34 +1001,19 @@ extern "C" int moddit_sparse_attn_fwd_scatter(const void* q, const void* k, cons
                                               int kv_len_lo, int kv_len_hi, void* const* peer_out, int n_peers,
                                               int head_base, float* lse, int32_t* status, void* stream) {
   clear_error();
+  MODDIT_CHECK_ARG(peer_out, "sparse_attn_fwd_scatter: null peer table");
+  MODDIT_CHECK_ARG(n_peers >= 1 && n_peers <= kMaxPeers, "sparse_attn_fwd_scatter: n_peers=%d outside [1, %d]", n_peers,
+                   kMaxPeers);
+  MODDIT_CHECK_ARG(N % n_peers == 0, "sparse_attn_fwd_scatter: N=%d does not divide over %d peers", N, n_peers);
+  MODDIT_CHECK_ARG(head_base >= 0, "sparse_attn_fwd_scatter: head_base must be non-negative");
   OutScatter sc = {};
-  if (int rc = make_scatter(&sc, peer_out, n_peers, head_base, N)) return rc;
-  return sparse_attn_dispatch(q, k, v, dtype, BH, N, D, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                              kv_len_hi, nullptr, lse, status, sc, nullptr, stream);
-}
-
-extern "C" size_t moddit_sparse_attn_fwd_split_bytes(int BH, int N, int D) {
-  if (BH <= 0 || N <= 0 || (D != 64 && D != 128)) return 0;
-  if ((ceil_div(N, kTile) + 1) / 2 > kSplitPairs) return 0;
-  return sizeof(float) * static_cast<size_t>(BH) * kLongPairs * kMaxParts * 256 * (D + 2);
-}
-
-extern "C" int moddit_sparse_attn_fwd_split(const void* q, const void* k, const void* v, int dtype, int BH, int N, int D,
-                                            const int32_t* counts, const int32_t* entries, const int32_t* order, int Hm,
-                                            float softmax_scale, int q_split, int kv_len_lo, int kv_len_hi, void* out,
-                                            void* const* peer_out, int n_peers, int head_base, float* lse, int32_t* status,
-                                            void* workspace, size_t workspace_bytes, void* stream) {
-  clear_error();
-  OutScatter sc = {};
-  if (n_peers > 0) {
-    if (int rc = make_scatter(&sc, peer_out, n_peers, head_base, N)) return rc;
-  } else {
-    MODDIT_CHECK_ARG(out, "sparse_attn_fwd_split: null output pointer");
+  for (int i = 0; i < n_peers; ++i) {
+    MODDIT_CHECK_ARG(peer_out[i] && aligned16(peer_out[i]), "sparse_attn_fwd_scatter: peer buffer %d null or unaligned", i);
+    sc.peer[i] = peer_out[i];
   }
-  const size_t need = moddit_sparse_attn_fwd_split_bytes(BH, N, D);
-  if (need > 0 && (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)))
-    return fail(MODDIT_E_WORKSPACE, "sparse_attn_fwd_split: %zu bytes of 16-byte aligned workspace needed", need);
+  sc.n_peers = n_peers;
+  sc.rows_per_peer = N / n_peers;
+  sc.head_base = head_base;
   return sparse_attn_dispatch(q, k, v, dtype, BH, N, D, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                              kv_len_hi, n_peers > 0 ? nullptr : out, lse, status, sc,
-                              need > 0 ? static_cast<float*>(workspace) : nullptr, stream);
+                              kv_len_hi, nullptr, lse, status, sc, stream);
 }

@@ -84,10 +84,6 @@ SIGNATURES = {
     "moddit_sparse_attn_fwd_scatter": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                                c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_int, c_void_p,
                                                c_int, c_int, c_void_p, c_void_p, c_void_p]),
-    "moddit_sparse_attn_fwd_split_bytes": (c_size_t, [c_int, c_int, c_int]),
-    "moddit_sparse_attn_fwd_split": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
-                                             c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_int, c_void_p,
-                                             c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "moddit_sparse_attn_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                        c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p,
                                        c_void_p, c_void_p]),
