@@ -98,6 +98,8 @@ int moddit_pooled_map_ws(const float* qbar, const float* kbar, int BH, int nb, i
  * :41-169) and the Triton twin MoD/mod/triton_flash_sparsity.py:28-98,181-225.
  *   q,k : (BH, N, D); lse : (BH, N) float32 natural log; map : (BH, n, n) float16
  *   map = count(S[r,c] < lse[r] + log_threshold) / block_size^2 with S = round_dtype(q*scale) k^T.
+ * Video regions past 539,904 tokens (4,218 tiles of 128) at head dimension 128 and 1,195,264 (9,338) at 64 return
+ * MODDIT_E_UNSUPPORTED.
  */
 int moddit_replay_map(const void* q, const void* k, const float* lse, int dtype, int BH, int N, int D,
                       int block_size, float softmax_scale, float log_threshold, int q_video_offset,

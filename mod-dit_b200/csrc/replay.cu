@@ -57,43 +57,52 @@ constexpr size_t smem_bytes() {
   return static_cast<size_t>(2 + kStages) * kTile * D * 2 + 1024 + sizeof(Control);
 }
 
-// What one CTA works on, as segments: whole query tiles in rounds over the grid while there is one for every CTA (CTAs
-// that run side by side stay on one head, whose K tiles they share through the L2), then its share of the tiles left over.
+// What one CTA works on, as segments: whole query tiles in rounds over the grid (CTAs that run side by side stay on one
+// head, whose K tiles they share through the L2), then its share of the tiles left over after whole rounds.  Left-over
+// tiles for four fifths of the grid or more are a round of their own: dealing them out would save a fifth of a tile's
+// sweep at most and costs a second segment's Q tile (16 heads of 9 x 9 tiles: 10.3 us, dealt out 12.3).
+// 32-bit throughout: the host admits items (heads x query tiles) below 2^31, and fewer than a grid are left over.
+// (64-bit divisions at every segment took 1-3 % of a launch.)
 struct Segments {
-  int pairs, ntk, rounds;
-  long long r;
-  int u;
+  int pairs, ntk, rounds, r, u;
   int bh, qt, p0, p1;      // current segment: pairs [p0, p1) of query tile qt of head bh
   __device__ __forceinline__ Segments(int BH, int ntk_) : pairs((ntk_ + 1) / 2), ntk(ntk_) {
-    const long long items = static_cast<long long>(BH) * ntk_;
+    const unsigned items = static_cast<unsigned>(BH) * ntk_;
     rounds = static_cast<int>(items / gridDim.x);
-    const long long tail0 = static_cast<long long>(rounds) * gridDim.x * pairs;
-    const long long tail = items * pairs - tail0;
+    unsigned left = items - rounds * gridDim.x;
+    tail0_ = items - left;
+    if (5 * left >= 4 * gridDim.x) {
+      if (blockIdx.x < left) ++rounds;
+      left = 0;
+    }
+    const unsigned units = left * pairs;
     r = 0;
     u = 0;
-    tail_u_ = tail0 + tail * blockIdx.x / gridDim.x;
-    tail_end_ = tail0 + tail * (blockIdx.x + 1) / gridDim.x;
+    tail_u_ = units * blockIdx.x / gridDim.x;
+    tail_end_ = units * (blockIdx.x + 1) / gridDim.x;
   }
   __device__ __forceinline__ bool next() {
+    unsigned item;
     if (r < rounds) {
-      item_ = r * gridDim.x + blockIdx.x;
+      item = static_cast<unsigned>(r) * gridDim.x + blockIdx.x;
       p0 = u;
       p1 = min(pairs, p0 + kSegPairs);
       u = p1;
       if (u == pairs) { u = 0; ++r; }
     } else {
       if (tail_u_ >= tail_end_) return false;
-      item_ = tail_u_ / pairs;
-      p0 = static_cast<int>(tail_u_ - item_ * pairs);
-      p1 = static_cast<int>(min(static_cast<long long>(min(pairs, p0 + kSegPairs)), p0 + (tail_end_ - tail_u_)));
+      const unsigned t = tail_u_ / pairs;
+      item = tail0_ + t;
+      p0 = static_cast<int>(tail_u_ - t * pairs);
+      p1 = min(min(pairs, p0 + kSegPairs), p0 + static_cast<int>(tail_end_ - tail_u_));
       tail_u_ += p1 - p0;
     }
-    bh = static_cast<int>(item_ / ntk);
-    qt = static_cast<int>(item_ - static_cast<long long>(bh) * ntk);
+    bh = static_cast<int>(item / ntk);
+    qt = static_cast<int>(item - static_cast<unsigned>(bh) * ntk);
     return true;
   }
  private:
-  long long item_, tail_u_, tail_end_;
+  unsigned tail0_, tail_u_, tail_end_;
 };
 
 __device__ __forceinline__ void report(int32_t* status, int code, int role, int where) {
@@ -235,10 +244,12 @@ __global__ void __launch_bounds__(kThreads, 1) replay_map_kernel(
       }
     }
   } else if (warp < 4) {
-    // scale + round each Q tile in place (element-wise, so the swizzled order does not matter)
+    // scale + round each Q tile in place (element-wise, so the swizzled order does not matter).  These warps wait through
+    // most of a sweep, beside count warps that bound the kernel: polling without sleep cost 48 heads of 352 x 352 tiles
+    // at head dimension 64 5 % (17.0 against 16.2 ms).
     bool ok = true;
     for (int sn = 0; ok && seg.next(); ++sn) {
-      ok = ptx::mbar_wait(bar(kQFull0 + (sn & 1)), (sn >> 1) & 1, abort_flag);
+      ok = ptx::mbar_wait_idle(bar(kQFull0 + (sn & 1)), (sn >> 1) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) { if (lane == 0) report(status, 4, 2, -1); break; }
       uint4* q4 = reinterpret_cast<uint4*>(smem + (sn & 1) * kTileBytes);
@@ -355,9 +366,9 @@ int launch(const void* q, const void* k, const float* lse, int dtype, int BH, in
   int sms = 0;
   if (int rc = sm_count(&sms)) return rc;
   const size_t smem = smem_bytes<D>();
-  // documented limit of this entry point: 4218 key tiles at head_dim 128, 9338 at 64
+  // the entry point's limit (moddit.h); with BH <= 65535 it keeps the item counts of Segments in 32 bits
   if (ntk > (D == 128 ? 4218 : 9338))
-    return fail(MODDIT_E_UNSUPPORTED, "replay_map: %d key tiles exceed the %d this kernel takes", ntk, D == 128 ? 4218 : 9338);
+    return fail(MODDIT_E_UNSUPPORTED, "replay_map: %d key tiles of 128 exceed the limit of %d", ntk, D == 128 ? 4218 : 9338);
   auto kernel = replay_map_kernel<D, kBF16>;
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   kernel<<<static_cast<unsigned>(units < sms ? units : sms), kThreads, smem, st>>>(tq, tk, lse, BH, N, bs, scale, log_thr, q_off, k_off, n,
