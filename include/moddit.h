@@ -289,7 +289,8 @@ int moddit_order_pairs(const int32_t* counts, int Hm, int npairs, int heads_per_
 /* The stages from moddit_pool_blocks to moddit_tile_lists in one call, for a step that predicts its mask from this
  * step's q and k (the pooled producer) and the features of the step before; every output equals what the single entry
  * points give.
- *   first, n  : video region in blocks: blocks [first, first + n) of ceil(N / block_size)
+ *   first, n  : video region in blocks: blocks [first, first + n) of nb = ceil(N / block_size); wan: first = 0, n = nb;
+ *               hunyuan: first = 0; cogvideox: first + n = nb; anything else is MODDIT_E_ARG
  *   factor    : from moddit_solve_small_prepare (small_solve != 0) or moddit_solve_prepare, regularization 1
  *   last_c/d  : features of the step before; d, c, b_d, modes, map_f16 receive this step's
  *   mask, counts, entries, order : as moddit_mask_from_lines / moddit_tile_lists write them

@@ -53,8 +53,18 @@ extern "C" int moddit_predict_lines(const void* q, const void* k, int dtype, int
   if (block_size != 64 && block_size != 128)
     return fail(MODDIT_E_UNSUPPORTED, "predict_lines: block_size must be 64 or 128, got %d", block_size);
   const int nb = ceil_div(N, block_size);
-  MODDIT_CHECK_ARG(first >= 0 && first + n <= nb, "predict_lines: video region [%d, %d + %d) exceeds %d blocks", first, first,
-                   n, nb);
+  MODDIT_CHECK_ARG(first >= 0 && n <= nb && first <= nb - n, "predict_lines: video region [%d, %d + %d) exceeds %d blocks",
+                   first, first, n, nb);
+  // The mask stage places the video region by its layout alone, and the list stage reads nb x nb blocks of what it wrote.
+  if (mask_layout == MODDIT_LAYOUT_WAN) {
+    MODDIT_CHECK_ARG(first == 0 && n == nb, "predict_lines: wan layout needs first == 0 and n == %d (got %d, %d)", nb, first, n);
+  } else if (mask_layout == MODDIT_LAYOUT_HUNYUAN) {
+    MODDIT_CHECK_ARG(first == 0, "predict_lines: hunyuan layout needs first == 0 (got %d)", first);
+  } else if (mask_layout == MODDIT_LAYOUT_COGVIDEOX) {
+    MODDIT_CHECK_ARG(first + n == nb, "predict_lines: cogvideox layout needs first + n == %d (got %d, %d)", nb, first, n);
+  } else {
+    return fail(MODDIT_E_ARG, "predict_lines: unknown layout %d", mask_layout);
+  }
   const Scratch s = layout(H, nb, D, n, top_k, small_solve != 0);
   if (workspace == nullptr || workspace_bytes < s.total || !aligned16(workspace))
     return fail(MODDIT_E_WORKSPACE, "predict_lines: %zu bytes of 16-byte aligned workspace needed", s.total);

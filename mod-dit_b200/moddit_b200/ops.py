@@ -664,17 +664,21 @@ def predict_lines(q: torch.Tensor, k: torch.Tensor, block_size: int, *, first: i
 
     Returns (map (H,n,n) float16, {'d', 'c', 'b_d'}, modes, mask, TileLists), each equal to what `pool_blocks`,
     `pooled_map`, `mts`, `solve`, `split_solution`, `select_lines`, `mask_from_lines` and `tile_lists` give."""
-    dev = _need_cuda(q, k, last['c'], last['d'])
-    _need_contig(q=q, k=k)
     if q.shape != k.shape or q.dtype != k.dtype or q.dim() != 4 or q.shape[0] != 1:
         raise ValueError("query and key must be (1, H, N, D) tensors of one dtype")
     if model_type not in _lib.LAYOUT:
         raise ValueError(f"Unknown model_type: {model_type}, expected 'wan', 'hunyuan', or 'cogvideox'")
     _, H, N, D = q.shape
+    nb = (N + block_size - 1) // block_size
+    if first < 0 or n < 1 or first + n > nb:
+        raise ValueError(f"video region [{first}, {first} + {n}) exceeds {nb} blocks")
+    if {"wan": first > 0 or n < nb, "hunyuan": first > 0, "cogvideox": first + n < nb}[model_type]:
+        raise ValueError(f"the {model_type} layout has no video region [{first}, {first} + {n}) in {nb} blocks")
+    dev = _need_cuda(q, k, last['c'], last['d'])
+    _need_contig(q=q, k=k)
     last_c, last_d = (last[key].to(torch.float32).contiguous() for key in ('c', 'd'))
     if tuple(last_c.shape) != (H, n) or tuple(last_d.shape) != (H, 2 * n - 1):
         raise ValueError("feature shapes must be c:(H,n) d:(H,2n-1)")
-    nb = (N + block_size - 1) // block_size
     ntq = (N + 127) // 128
     npairs = (ntq + 1) // 2
     nbt = n if model_type == "wan" else nb

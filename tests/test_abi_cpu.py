@@ -70,3 +70,26 @@ def test_work_lists_survive_pickling_with_the_state_dict():
     counts, entries = back["_tile_lists"][1]
     assert torch.equal(counts, lists.counts) and torch.equal(entries, lists.entries)
     assert torch.equal(back["_tile_lists"][1].order, lists.order)
+
+
+@pytest.mark.parametrize("layout,first,n,nb,text", [("wan", 0, 7, 8, b"wan"), ("wan", 1, 7, 8, b"wan"),
+                                                    ("hunyuan", 1, 6, 8, b"hunyuan"), ("hunyuan", 2, 6, 8, b"hunyuan"),
+                                                    ("cogvideox", 1, 6, 8, b"cogvideox"), ("cogvideox", 0, 7, 8, b"cogvideox"),
+                                                    ("wan", 0, 9, 8, b"exceeds"), (None, 0, 8, 8, b"layout")])
+def test_prediction_refuses_a_video_region_that_the_layout_does_not_have(layout, first, n, nb, text):
+    """The mask of the wan layout covers n blocks and the work lists are built over all of them, so n short of the
+    sequence would be read past the mask; the other layouts put their video blocks at one place only."""
+    from moddit_b200 import _lib, ops
+    lib = _lib.lib
+    buf = ctypes.create_string_buffer(64)
+    p = ctypes.c_void_p((ctypes.addressof(buf) + 15) // 16 * 16)
+    N = 64 * nb - 5
+    code = 9 if layout is None else _lib.LAYOUT[layout]
+    rc = lib.moddit_predict_lines(p, p, 0, 2, N, 64, 64, first, n, 2, code, 0.125, p, 1, p, p, 3, 5.0, 1.0, p, p, p, p, p,
+                                  p, p, p, None, p, 1 << 40, None)
+    assert rc == -1 and text in lib.moddit_last_error_string()
+    q = torch.zeros(1, 2, N, 64, dtype=torch.bfloat16)
+    last = {"c": torch.zeros(2, n), "d": torch.zeros(2, 2 * n - 1)}
+    with pytest.raises(ValueError, match="video region|model_type"):
+        ops.predict_lines(q, q, 64, first=first, n=n, blocks_per_frame=2, model_type=layout or "other", last=last, top_k=3,
+                          predict_T=5)
