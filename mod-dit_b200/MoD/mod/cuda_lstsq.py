@@ -43,7 +43,8 @@ def reconstruct_attention_map(features, n, blocks_per_frame=4):
 
 def features_from_solution(X: torch.Tensor, n: int):
     """Split the raw solution (H, 3n) as MoD/mod/cuda_lstsq.py:257-261 does ('c' is halved)."""
-    return _ops.split_solution(X, n)[0]
+    nd = 2 * n - 1
+    return {'d': X[:, :nd], 'c': X[:, nd:nd + n] / 2, 'b_d': X[:, -1]}
 
 
 def solve_lstsq(warmup_state, S_T, step, blocks_per_frame, layer_idx=0, regularization=1e-5, use_cuda=True):
