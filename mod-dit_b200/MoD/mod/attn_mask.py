@@ -581,14 +581,15 @@ def _spargeattn_step(query, key, value, warmup_state):
 
 def _predicts_in_one_call(query, warmup_state, history, current_step) -> bool:
     """Whether a step's prediction is the plain line prediction of one sequence, which is a single call; stages that are
-    being timed one by one, work lists ordered by groups of heads and the other selector go stage by stage."""
+    being timed one by one or shown as NVTX ranges, work lists ordered by groups of heads and the other selector go stage
+    by stage."""
     return (bool(history) and current_step != warmup_state['warmup_steps'] - 2
             and query.shape[0] == 1 and warmup_state['model_type'] in _lib.LAYOUT
             and warmup_state.get('selector', 'topk_lines') != 'cumulative_mass'
             and int(warmup_state.get('_head_groups') or 1) <= 1
             and tuple(history[-1]['c'].shape) == (query.shape[1], _geometry(warmup_state, query.shape[2])[1])
             and history[-1]['c'].device == query.device
-            and not _ops.timing_active("moddit_pool_blocks"))
+            and not _ops.watched_by_stage())
 
 
 def _pooled_step(query, key, value, warmup_state, logger, pre_defined_mask, current_step, layer_idx,

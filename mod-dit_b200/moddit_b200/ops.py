@@ -21,7 +21,7 @@ _DTYPE = {torch.bfloat16: _lib.MODDIT_BF16, torch.float16: _lib.MODDIT_FP16}
 # ---------------------------------------------------------------------------------------------
 # optional per-entry-point timing (CUDA events on the launching stream); off by default
 # ---------------------------------------------------------------------------------------------
-_TIMING = {"on": False, "only": None, "records": [], "launches": 0,
+_TIMING = {"on": False, "only": None, "by_stage": True, "records": [], "launches": 0,
            "nvtx": os.environ.get("MODDIT_NVTX", "0") not in ("", "0")}
 # kernels launched by one call of each entry point (for launch accounting in benchmarks)
 KERNELS_PER_CALL = {"moddit_pool_blocks": 1, "moddit_pooled_map": 1, "moddit_pooled_map_ws": 3, "moddit_replay_map": 1,
@@ -34,10 +34,13 @@ KERNELS_PER_CALL = {"moddit_pool_blocks": 1, "moddit_pooled_map": 1, "moddit_poo
                     "moddit_mts_noalloc": 2, "moddit_copy_rows_dma": 0, "moddit_qkv_prologue": 1}
 
 
-def stage_timing(enable: bool, only=None) -> None:
+def stage_timing(enable: bool, only=None, by_stage: bool = True) -> None:
     """Turn launch counting and event timing of the entry-point calls on or off and clear the records.
-    `only`: names of the entry points to time (all when None); the others are still counted."""
+    `only`: names of the entry points to time (all when None); the others are still counted.
+    by_stage: steps run a prediction as single calls, one record each; False leaves them on the path that they take
+    when nothing is timed (one call, one record)."""
     _TIMING["on"] = bool(enable)
+    _TIMING["by_stage"] = bool(by_stage)
     _TIMING["only"] = None if only is None else frozenset(only)
     _TIMING["records"] = []
     _TIMING["launches"] = 0
@@ -57,6 +60,12 @@ def stage_records():
 
 def launches_recorded() -> int:
     return _TIMING["launches"]
+
+
+def watched_by_stage() -> bool:
+    """Whether someone looks at the single stages of a prediction (NVTX ranges, or timing of stage by stage), so that
+    a step has to run them as calls of their own."""
+    return bool(_TIMING["nvtx"]) or (_TIMING["by_stage"] and timing_active("moddit_pool_blocks"))
 
 
 def timing_active(name: str) -> bool:
