@@ -431,12 +431,16 @@ def run_ours(args):
     breakdown_steps = max(1, min(args.steps, 5))
     # one more step goes first, unrecorded: its attention kernel keeps the GPU busy while the host enqueues the
     # recorded steps, so that the events bracket kernels waiting in the queue and not the host's launch latency
-    layer(q_in, k_in, v_in, step_no)
-    ops.stage_timing(True)
-    for i in range(breakdown_steps):
-        layer(q_in, k_in, v_in, step_no + 1 + i)
-    records = ops.stage_records()
-    ops.stage_timing(False)
+    # Two passes: the prediction on the path that a step takes (mask_pred_ms), then as single calls (stage_ms_per_step).
+    recorded = []
+    for by_stage in (False, True):
+        layer(q_in, k_in, v_in, step_no)
+        ops.stage_timing(True, by_stage=by_stage)
+        for i in range(breakdown_steps):
+            layer(q_in, k_in, v_in, step_no + 1 + i)
+        recorded.append(ops.stage_records())
+        ops.stage_timing(False)
+        step_no += 1 + breakdown_steps
     ops.check_health(dev)
     timeline = None
     if args.timeline and world > 1 and hx.head_groups() == 1 and hx.resharder is not None:
@@ -462,12 +466,13 @@ def run_ours(args):
     flops_local = kept_flops(mask, bs, D)
     per_head = 1.0 - mask.float().mean(dim=(1, 2))
     sparsity_local = float(per_head.mean().item())
-    stage_ms = {}
-    for name, ms in records:
-        stage_ms[name] = stage_ms.get(name, 0.0) + ms
+    path_ms, stage_ms = {}, {}
+    for total, records in zip((path_ms, stage_ms), recorded):
+        for name, ms in records:
+            total[name] = total.get(name, 0.0) + ms
     copies = ("moddit_copy_rows", "moddit_copy_rows_dma")               # re-shard copies (N > 1 only)
-    comm_ms = sum(stage_ms.get(name, 0.0) for name in copies) / breakdown_steps
-    pred_ms = sum(ms for name, ms in stage_ms.items()
+    comm_ms = sum(path_ms.get(name, 0.0) for name in copies) / breakdown_steps
+    pred_ms = sum(ms for name, ms in path_ms.items()
                   if name not in ("moddit_sparse_attn_fwd",) + copies) / breakdown_steps
 
     # ---- e2e: inputs in pinned host memory, output copied back ----------------------------------
@@ -653,7 +658,7 @@ def run_sweep(args):
         else:
             regime = "dense" if step == 0 else "sparse"      # the first call has no feature history yet
         hx.barrier()
-        ops.stage_timing(True)
+        ops.stage_timing(True, by_stage=False)
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         # A step is timed alone (its inputs are new), so the GPU would sit idle while the host enqueues the step's
         # launches one by one and the events would measure the host.  A few milliseconds of busy-waiting on the
