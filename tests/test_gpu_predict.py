@@ -12,7 +12,10 @@ def ops():
 
 
 @pytest.mark.parametrize("model,D,bs,grid,text", [("wan", 64, 64, (4, 32, 32), 0), ("hunyuan", 128, 128, (6, 32, 48), 200),
-                                                  ("cogvideox", 64, 64, (3, 33, 41), 130)])
+                                                  ("cogvideox", 64, 64, (3, 33, 41), 130),
+                                                  # past the sizes of the small solve: n = 96, 120 and 106
+                                                  ("wan", 128, 64, (6, 32, 32), 0), ("hunyuan", 128, 128, (10, 32, 48), 200),
+                                                  ("cogvideox", 64, 64, (5, 33, 41), 130)])
 def test_prediction_in_one_call_equals_the_stages(ops, model, D, bs, grid, text):
     from moddit_b200 import _lib, synth
     from MoD.mod.attn_mask import block_geometry
@@ -41,3 +44,28 @@ def test_prediction_in_one_call_equals_the_stages(ops, model, D, bs, grid, text)
     assert torch.equal(got[4].counts, lists.counts) and torch.equal(got[4].order, lists.order)
     live = torch.arange(lists.entries.shape[-1], device="cuda") < lists.counts[..., None]
     assert torch.equal(got[4].entries[live], lists.entries[live])
+
+
+@pytest.mark.parametrize("model,grid,text", [("wan", (4, 32, 32), 0), ("cogvideox", (5, 33, 41), 130)])
+def test_watched_step_equals_the_unwatched_one(ops, model, grid, text):
+    """A layer's step gives the same output and state whether its prediction is one call or, under timing, single ones."""
+    import logging
+    from moddit_b200 import synth
+    from MoD.mod.attn_mask import SparseAttentionWithMap
+    from MoD.mod.state import create_adaptive_mask_state
+    H, video = 2, grid[0] * grid[1] * grid[2]
+    got = []
+    for watched in (False, True):
+        state = create_adaptive_mask_state(model, H, video, text, grid[1] * grid[2], grid[0], warmup_steps=2, top_k=12,
+                                           predict_T=5, block_size=64)
+        state["score_producer"] = "pooled"
+        ops.stage_timing(watched)
+        for step in range(4):
+            q, k, v = synth.make_qkv(heads=H, grid=grid, head_dim=64, text_tokens=text, text_first=model == "cogvideox",
+                                     seed=20 + step, device="cuda")
+            out, _ = SparseAttentionWithMap(q, k, v, state, logging.getLogger("test"), current_step=step)
+        names = [name for name, _ in ops.stage_records()]
+        ops.stage_timing(False)
+        assert watched == ("moddit_pool_blocks" in names)
+        got.append((out, state["mask"], state["prev_full_maps"], state["mode"], *state["features_history"][-1].values()))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
