@@ -7,9 +7,8 @@
 // back to back on constant shared-memory / tensor-memory operands and the elapsed SM clocks per MMA are printed,
 // for N = 64 / 128 / 256, both operands in shared memory (SS) or A in tensor memory (TS), with and without a
 // tcgen05.commit after every group, with extra (already complete) mbarrier waits per group, and with the other
-// warps of the CTA busy on the FMA / special-function pipes.  It explains the ceiling of the sparse forward's
-// single issuing thread: the pipe needs 64 clocks for an N = 128 product, the issuing warp can hand one over
-// only every ~84.  Every wait is bounded (ptx::mbar_wait).
+// warps of the CTA busy on the FMA / special-function pipes; each once with the issuing thread picked by
+// `lane == 0` and once by elect.sync.  Every wait is bounded (ptx::mbar_wait).
 #include <cstdio>
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -19,14 +18,14 @@ using namespace moddit;
 struct Res { long long clks; int err; };
 
 // KIND: 0 SS N128, 1 SS N256, 2 TS N128, 3 SS N64, 4 TS N64, 5 TS N256
-template <int KIND>
+template <int KIND, bool ELECT>
 __global__ void __launch_bounds__(384, 1) bench(Res* res, int reps, int commit_every, int issuers, int noise, int waits_per_group) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ unsigned long long bars[4];
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = ELECT ? ptx::warp_index() : static_cast<int>(threadIdx.x / 32), lane = threadIdx.x % 32;
   constexpr int N = (KIND == 1 || KIND == 5) ? 256 : ((KIND == 3 || KIND == 4) ? 64 : 128);
   constexpr bool TS = (KIND == 2 || KIND == 4 || KIND == 5);
   const uint32_t sA = ptx::smem_u32(smem);              // 128 x 128 bf16 = 32 KB
@@ -43,7 +42,7 @@ __global__ void __launch_bounds__(384, 1) bench(Res* res, int reps, int commit_e
   ptx::tc_fence_after();
   const uint32_t tmem = tmem_base;
   volatile int* af = &abort_flag;
-  if (warp < issuers && lane == 0) {
+  if (warp < issuers && (ELECT ? ptx::elect_one() : lane == 0)) {
     const uint32_t idesc = ptx::idesc_f16(128, N, true, false);
     const uint64_t da = ptx::smem_desc_sw128(sA, 16, 1024);
     const uint64_t db = ptx::smem_desc_sw128(sB, 16, 1024);
@@ -89,36 +88,43 @@ __global__ void __launch_bounds__(384, 1) bench(Res* res, int reps, int commit_e
   if (warp == 2) { ptx::tc_fence_after(); ptx::tmem_dealloc(tmem, 512); }
 }
 
-template <int KIND>
+template <int KIND, bool ELECT>
 void run(const char* name, Res* d, int reps, int commit_every, int issuers, int noise, int waits) {
-  cudaFuncSetAttribute(bench<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+  cudaFuncSetAttribute(bench<KIND, ELECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
   cudaMemset(d, 0, sizeof(Res) * 4);
-  bench<KIND><<<148, 384, 100 * 1024>>>(d, reps, commit_every, issuers, noise, waits);
+  bench<KIND, ELECT><<<148, 384, 100 * 1024>>>(d, reps, commit_every, issuers, noise, waits);
   cudaError_t e = cudaDeviceSynchronize();
   Res h[4];
   cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
-  printf("%-10s commit_every=%-5d issuers=%d noise=%d waits=%d : %.1f clk/MMA (issuer0) %.1f (issuer1) err=%d/%d cuda=%s\n", name, commit_every,
+  printf("%-5s %-10s commit_every=%-5d issuers=%d noise=%d waits=%d : %.1f clk/MMA (issuer0) %.1f (issuer1) err=%d/%d cuda=%s\n", ELECT ? "elect" : "lane0", name, commit_every,
          issuers, noise, waits, (double)h[0].clks / (8.0 * reps), (double)h[1].clks / (8.0 * reps), h[0].err, h[1].err, cudaGetErrorString(e));
 }
 
-int main() {
-  Res* d; cudaMalloc(&d, sizeof(Res) * 4);
+template <bool E>
+void all(Res* d) {
   const int R = 2000;
   for (int ce : {0, 1}) {
-    run<0>("SS N128", d, R, ce, 1, 0, 0);
-    run<1>("SS N256", d, R, ce, 1, 0, 0);
-    run<3>("SS N64", d, R, ce, 1, 0, 0);
-    run<2>("TS N128", d, R, ce, 1, 0, 0);
-    run<5>("TS N256", d, R, ce, 1, 0, 0);
-    run<4>("TS N64", d, R, ce, 1, 0, 0);
+    run<0, E>("SS N128", d, R, ce, 1, 0, 0);
+    run<1, E>("SS N256", d, R, ce, 1, 0, 0);
+    run<3, E>("SS N64", d, R, ce, 1, 0, 0);
+    run<2, E>("TS N128", d, R, ce, 1, 0, 0);
+    run<5, E>("TS N256", d, R, ce, 1, 0, 0);
+    run<4, E>("TS N64", d, R, ce, 1, 0, 0);
   }
-  run<0>("SS N128", d, R, 1, 2, 0, 0);
-  run<2>("TS N128", d, R, 1, 2, 0, 0);
-  run<0>("SS N128", d, R, 1, 1, 4, 0);
-  run<2>("TS N128", d, R, 1, 1, 4, 0);
-  run<0>("SS N128", d, R, 1, 1, 0, 1);
-  run<0>("SS N128", d, R, 1, 1, 0, 2);
-  run<2>("TS N128", d, R, 1, 1, 0, 2);
-  run<0>("SS N128", d, R, 1, 1, 4, 2);
+  run<0, E>("SS N128", d, R, 1, 2, 0, 0);
+  run<2, E>("TS N128", d, R, 1, 2, 0, 0);
+  run<0, E>("SS N128", d, R, 1, 1, 4, 0);
+  run<2, E>("TS N128", d, R, 1, 1, 4, 0);
+  run<0, E>("SS N128", d, R, 1, 1, 0, 1);
+  run<0, E>("SS N128", d, R, 1, 1, 0, 2);
+  run<2, E>("TS N128", d, R, 1, 1, 0, 2);
+  run<0, E>("SS N128", d, R, 1, 1, 4, 2);
+}
+
+int main() {
+  Res* d;
+  cudaMalloc(&d, sizeof(Res) * 4);
+  all<false>(d);
+  all<true>(d);
   return 0;
 }

@@ -14,9 +14,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// True in one thread of a converged warp.  The compiler knows that at most one thread is active behind it, so a
-// tcgen05.mma takes its descriptors straight from uniform registers; behind a `lane == 0` test every instruction goes
-// through a loop over the active threads.
+// True in one thread of a converged warp.  Measured on back-to-back M128 x N128 x K16 products (64 clocks of tensor pipe
+// each): a thread picked this way hands one over every 64 clocks, one picked by `lane == 0` every 84; with a
+// tcgen05.commit after every eight, 67 against 113 (benchmarks/mma_issue_bench.cu).
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;
   asm volatile(
@@ -237,11 +237,6 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   return r;
 }
 // a * b + c clamped to [0, 1]
-__device__ __forceinline__ float fma_sat(float a, float b, float c) {
-  float r;
-  asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));

@@ -144,13 +144,12 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
   const uint32_t tmem = ctl->tmem_base;
 
   // Register budget: the softmax warpgroups hold a 128-value row per thread, the control warps need little
-  // (128 control threads give up what 256 softmax threads take: 168 -> 72 / 216 at D = 128 and 56 / 224 at
-  // D = 64, the splits that leave each instantiation without a single spill).
+  // (128 control threads give up what 256 softmax threads take: 168 -> 72 / 216, the split that leaves each
+  // instantiation without a spill).
   // The control branch and the softmax branch are disjoint in the control-flow graph so that each gets
   // its own register allocation.
   if (warp < 4) {
-  if constexpr (D == 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-  else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (ptx::elect_one()) {
@@ -278,8 +277,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
     }
   }
   } else {
-    if constexpr (D == 128) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
-    else asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     // ------------------------------------------------------------------ softmax + epilogue
     const int x = (warp - 4) / 4;                 // 0: tile A, 1: tile B
     const int wq = warp % 4;                      // tensor-memory lane quarter of this warp
@@ -355,8 +353,8 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
       }
       // P = exp2(S*scale - m), two fp32 lanes per instruction where the hardware has packed forms.  The row is handed to
       // the MMA warp in two parts, P*V of the first running while the second is still being computed: 96 keys, then 32,
-      // so that only two of the eight products are left when the row is done (halves left four: HunyuanVideo launch
-      // 20.36 -> 20.02 ms, four heads over 8,448 tokens 134 -> 132 us).
+      // so that only two of the eight products are left when the row is done (halves left four; both in turn in one
+      // process: HunyuanVideo launch 20.76 -> 20.50 ms, Wan 15.35 -> 15.07, four heads over 8,448 tokens 115 -> 111 us).
       const float ref = (m == -INFINITY) ? 0.f : m;
       const uint64_t scale2 = ptx::pack_f32x2(scale_log2, scale_log2);
       const uint64_t nref2 = ptx::pack_f32x2(-ref, -ref);
@@ -395,8 +393,6 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
       ++done;
     }
 
-    if (lane == 0 && wq == 0) {
-    }
     if (ok) {
       ok = ptx::mbar_wait(bar(kOFinal), 0, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
@@ -462,8 +458,11 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
 // P has columns of its own, so Q K^T of the NEXT entry is issued as soon as the softmax has read S of the current
 // one into registers (barrier kSFree), and a tile's softmax runs back to back while its products run beside it.
 // With the chain gone the two query tiles no longer need one thread to hold them in anti-phase, and each tile gets
-// its own issuing thread (warps 1 and 3: a warp can hand over one tcgen05.mma per ~84 clocks, and the twelve
-// instructions of a tile-entry at this size keep the pipe busy for half of that).
+// its own issuing thread (warps 1 and 3).
+// What bounds it: the softmax warps' chain of fixed latencies, two warps per scheduler.  With 16,640 tokens and 16
+// heads the exponential unit is busy 59 % of the time, the tensor pipe 33 %, issue slots are used 42 %, and the most
+// frequent stall is an instruction's fixed latency (2.1 warps per issue; by a full math pipe 0.11).
+// The floor is the exponential unit's 1024 clocks per tile.
 // What P V(X, e) must not overlap is (1) the softmax overwriting P_X with the next entry's values and (2) the softmax
 // rescaling O_X; both wait for tile X's issuer to have finished slot e (kDone_X, committed after the issuer's last
 // MMA of the slot), which is also what tells the producer that the slot's K/V stages are free (it waits for both
@@ -510,57 +509,17 @@ __device__ __forceinline__ float row_max64(const float* v) {
 }
 
 // P = exp2(S * scale - ref) for 64 columns of one row: pk[32] = 16-bit pairs; the row sum goes into the packed sums.
-//
-// The exponential unit does 16 results per clock and SM: a 128 x 128 tile of P costs it 1024 clocks, twice what the
-// tensor pipe needs for the tile's two products at D = 64, and with the chain between the products broken it is
-// the unit this kernel waits for.  kPoly of every 8 column pairs are therefore computed on the FMA pipe instead:
-//   2^x = 2^n * p(f),  n = round(x),  f = x - n in [-1/2, 1/2],  p a cubic with relative error 7.5e-5 (a sixth of
-// the rounding step of a bfloat16 P, a sixth of a float16 one's), 2^n added into the exponent field.  x is first
-// clamped to [-120, 8] by a saturating FMA ((x + 120) / 128 in [0, 1]); the upper end is the most the lazily
-// updated row maximum can trail by, and 2^-120 stands in for anything smaller - rows that must give exact zeros
-// (masked columns) use kPoly = 0.
-#ifndef MODDIT_D64_POLY_PAIRS
-#define MODDIT_D64_POLY_PAIRS 0
-#endif
-constexpr int kPolyPairs64 = MODDIT_D64_POLY_PAIRS;
-
-template <bool kBF16, int kPoly>
+template <bool kBF16>
 __device__ __forceinline__ void exp_half(const float* v, float scale_log2, float ref, uint32_t* pk, uint64_t& sum2a,
                                          uint64_t& sum2b) {
   const uint64_t scale2 = ptx::pack_f32x2(scale_log2, scale_log2);
   const uint64_t nref2 = ptx::pack_f32x2(-ref, -ref);
-  const float pa = scale_log2 * 0.0078125f;
-  const float pb = (120.f - ref) * 0.0078125f;
-  constexpr float kMagic = 12582912.f - 120.f;            // 1.5 * 2^23 - 120: adding it rounds to an integer
-  const uint64_t k128 = ptx::pack_f32x2(128.f, 128.f);
-  const uint64_t kmag = ptx::pack_f32x2(kMagic, kMagic);
-  const uint64_t kneg = ptx::pack_f32x2(-1.f, -1.f);
-  const uint64_t c3 = ptx::pack_f32x2(0.05517167f, 0.05517167f);
-  const uint64_t c2 = ptx::pack_f32x2(0.24261113f, 0.24261113f);
-  const uint64_t c1 = ptx::pack_f32x2(0.69326097f, 0.69326097f);
-  const uint64_t c0 = ptx::pack_f32x2(0.99992806f, 0.99992806f);
 #pragma unroll
   for (int i = 0; i < 32; ++i) {
-    float p0, p1;
-    if (((i % 8) * kPoly) % 8 < kPoly) {
-      const uint64_t y2 = ptx::pack_f32x2(ptx::fma_sat(v[2 * i], pa, pb), ptx::fma_sat(v[2 * i + 1], pa, pb));
-      const uint64_t r2 = ptx::fma_f32x2(y2, k128, kmag);         // x + 1.5 * 2^23: the integer n sits in the low bits
-      const uint64_t f2 = ptx::fma_f32x2(y2, k128, ptx::fma_f32x2(r2, kneg, kmag));   // x - n
-      uint64_t q2 = ptx::fma_f32x2(f2, c3, c2);
-      q2 = ptx::fma_f32x2(q2, f2, c1);
-      q2 = ptx::fma_f32x2(q2, f2, c0);
-      float r0, r1, q0, q1;
-      ptx::unpack_f32x2(r2, r0, r1);
-      ptx::unpack_f32x2(q2, q0, q1);
-      p0 = __uint_as_float(__float_as_uint(q0) + (__float_as_uint(r0) << 23));
-      p1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(r1) << 23));
-    } else {
-      const uint64_t x2 = ptx::fma_f32x2(ptx::pack_f32x2(v[2 * i], v[2 * i + 1]), scale2, nref2);
-      float x0, x1;
-      ptx::unpack_f32x2(x2, x0, x1);
-      p0 = ptx::ex2(x0);
-      p1 = ptx::ex2(x1);
-    }
+    const uint64_t x2 = ptx::fma_f32x2(ptx::pack_f32x2(v[2 * i], v[2 * i + 1]), scale2, nref2);
+    float x0, x1;
+    ptx::unpack_f32x2(x2, x0, x1);
+    const float p0 = ptx::ex2(x0), p1 = ptx::ex2(x1);
     const uint64_t p2 = ptx::pack_f32x2(p0, p1);
     if (i & 1) sum2b = ptx::add_f32x2(sum2b, p2); else sum2a = ptx::add_f32x2(sum2a, p2);
     pk[i] = pack2<kBF16>(p0, p1);
@@ -830,8 +789,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
       for (int half = 0; half < 2; ++half) {
         uint32_t pk[32];
         if (keep[half]) {
-          if (edge) exp_half<kBF16, 0>(v + half * 64, scale_log2, ref, pk, sum2a, sum2b);   // may hold -inf: exact zeros
-          else exp_half<kBF16, kPolyPairs64>(v + half * 64, scale_log2, ref, pk, sum2a, sum2b);
+          exp_half<kBF16>(v + half * 64, scale_log2, ref, pk, sum2a, sum2b);
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) pk[i] = 0u;   // a half this row half does not keep: no exponentials at all
@@ -971,17 +929,10 @@ static int sparse_attn_dispatch(const void* q, const void* k, const void* v, int
                : launch<128, false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
                                     kv_len_hi, out, lse, status, scatter, st);
   }
-#ifdef MODDIT_D64_SHARED_KERNEL
-  return dtype == MODDIT_BF16 ? launch<64, true>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
-                                                 kv_len_lo, kv_len_hi, out, lse, status, scatter, st)
-                              : launch<64, false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
-                                                  kv_len_lo, kv_len_hi, out, lse, status, scatter, st);
-#else
   return dtype == MODDIT_BF16 ? launch_d64<true>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
                                                  kv_len_lo, kv_len_hi, out, lse, status, scatter, st)
                               : launch_d64<false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
                                                   kv_len_lo, kv_len_hi, out, lse, status, scatter, st);
-#endif
 }
 
 extern "C" int moddit_sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype, int BH, int N, int D,
