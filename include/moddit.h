@@ -193,8 +193,8 @@ size_t moddit_solve_workspace_bytes(int H, int n);
 int moddit_solve(const float* mts, const void* factor, int H, int n, int blocks_per_frame,
                  double regularization, float* X, void* workspace, size_t workspace_bytes, void* stream);
 
-/* The same solve for small systems in the form the specification words it: the normal equations M^T M + reg*I
- * (3n x 3n, closed form) are built in one CTA's shared memory and inverted there in float64
+/* The same solve for small systems: the normal equations M^T M + reg*I (3n x 3n, closed form, diagonal + reg rounded to
+ * float32 as in moddit_mtm) are built in one CTA's shared memory and inverted there in float64
  * (moddit_solve_small_prepare, once per (n, blocks_per_frame, reg): the reference caches its factor the same way,
  * MoD/mod/cuda_lstsq.py:153-186); per call every unknown is the dot product of a row of that inverse with the head's
  * right-hand side, summed in float64 (moddit_solve_small).  It solves the system of the reference's

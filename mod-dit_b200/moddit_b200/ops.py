@@ -462,8 +462,8 @@ def _small_factor(n: int, blocks_per_frame: int, regularization: float, device) 
 
 
 def _takes_small_solve(n: int, regularization: float) -> bool:
-    """The float32-system route only for well-conditioned systems (the regularisation the path uses is 1; with a tiny
-    one the unregularised rank deficiency is a float32 pivot away)."""
+    """The small route only for regularisations that survive the rounding of a diagonal entry of up to n + regularization
+    to float32 (the path uses 1): M^T M is rank deficient, so its smallest eigenvalue is the regularization alone."""
     return n <= lib.moddit_solve_small_max_n() and regularization >= 0.5
 
 
@@ -472,9 +472,9 @@ def solve(mts_: torch.Tensor, n: int, blocks_per_frame: int, regularization: flo
     """X (H, 3n) float32 with (M^T M + regularization * I) X = mts.
 
     method "small": normal equations inverted in shared memory once per geometry, one product per call
-    (`moddit_solve_small`; n <= `lib.moddit_solve_small_max_n()`); "structured": the float64 structured elimination against a factor
-    cached per geometry (`moddit_solve`); "auto": "small" where it fits and regularization >= 0.5, else
-    "structured"."""
+    (`moddit_solve_small`; n <= `lib.moddit_solve_small_max_n()`); "structured": the float64 structured elimination
+    against a factor cached per geometry (`moddit_solve`); "auto": "small" where it fits and regularization >= 0.5,
+    else "structured"."""
     dev = _need_cuda(mts_)
     mts_ = mts_.contiguous()
     if mts_.dtype != torch.float32 or mts_.shape[1] != 3 * n:

@@ -181,9 +181,9 @@ def test_solve_matches_reference_golden(ops, golden_dir):
 
 @pytest.mark.parametrize("n,bpf,H", [(12, 4, 3), (13, 4, 9), (64, 16, 2), (74, 30, 17)])
 def test_small_solve_in_shared_memory_matches_the_exact_solve(ops, n, bpf, H):
-    """Normal equations in shared memory, float32 Cholesky, one warp per head (the specification's wording; what
-    `ops.solve` picks for n <= 74) against the oracle's float64 solve of the same system and against the structured
-    float64 route; n = 64 is the specification's first configuration, 17 heads need three CTAs."""
+    """Normal equations inverted in shared memory, one dot product per unknown (what `ops.solve` picks for n <= 74)
+    against the oracle's float64 solve of the same system and against the structured float64 route; n = 64 is the first
+    of the configurations, 17 heads are four whole groups of four and one head."""
     S = _grid_map(H, n, 64, 40 + n)
     mts = orc.compute_mts(S, bpf)
     ref = orc.solve_features(mts, n, bpf, 1.0, precise=True)
