@@ -451,37 +451,32 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
 // ====================================================================================================
 // Head dimension 64.
 //
-// At D = 64 a 128 x 128 tile carries half the tensor work of the D = 128 tile for the same 16,384 exponentials, so
-// the kernel above - in which a tile's chain Q K^T -> softmax -> P V is strictly serial because P overwrites S -
-// spends most of a key-tile slot waiting on that chain.  Here tensor memory has room to break the chain:
-//   S_A [0,128)  S_B [128,256)  O_A [256,320)  O_B [320,384)  P_A [384,448)  P_B [448,512)
-// P has columns of its own, so Q K^T of the NEXT entry is issued as soon as the softmax has read S of the current
-// one into registers (barrier kSFree), and a tile's softmax runs back to back while its products run beside it.
-// With the chain gone the two query tiles no longer need one thread to hold them in anti-phase, and each tile gets
-// its own issuing thread (warps 1 and 3).
-// What bounds it: the softmax warps' chain of fixed latencies, two warps per scheduler.  With 16,640 tokens and 16
-// heads the exponential unit is busy 59 % of the time, the tensor pipe 33 %, issue slots are used 42 %, and the most
-// frequent stall is an instruction's fixed latency (2.1 warps per issue; by a full math pipe 0.11).
-// The floor is the exponential unit's 1024 clocks per tile.
-// What P V(X, e) must not overlap is (1) the softmax overwriting P_X with the next entry's values and (2) the softmax
-// rescaling O_X; both wait for tile X's issuer to have finished slot e (kDone_X, committed after the issuer's last
-// MMA of the slot), which is also what tells the producer that the slot's K/V stages are free (it waits for both
-// tiles').  The barrier is per tile on purpose: one barrier for both would release the two tiles' exponentials at
-// the same instant, and they share the special-function unit.
+// At D = 64 a tile carries half the tensor work of the D = 128 tile for the same exponentials, and two softmax warps per
+// scheduler do not fill the exponential unit: with one warpgroup per query tile and 128-key rows a slot (two query tiles x
+// one key tile) took 3,100 clocks for 2,048 of that unit, both warps busy throughout with latencies of their own.  So every
+// query tile has two independent chains, one for either 64-key half of its key tiles: scores, online softmax with a
+// reference and a sum of its own, P V into an accumulator of its own - four warpgroups, four warps per scheduler, nothing
+// exchanged until the two accumulators of a row are put together at the end.
+//   S_c [64 c, 64 c + 64)   O_c [256 + 64 c, 320 + 64 c)   for chain c = 2 * tile + half; P_c (16-bit) overwrites the first
+//   32 columns of S_c.
+// Each query tile has an issuing thread that takes its two chains in turn, PV(0,e) QK(0,e+1) PV(1,e) QK(1,e+1): products of
+// one thread execute in order, which makes the aliasing of P and S safe and lets "S ready" imply that the chain's previous
+// P V is done.  A half that neither half of the tile's rows keeps costs nothing.
+// Measured, launch alone, before -> now: 48 heads x 45,104 tokens at 12 % of the blocks 4.82 -> 4.22 ms, 32 heads x 16,640
+// tokens at 33 % 1.21 -> 1.07, dense 48 heads x 20,624 tokens 7.2 -> 6.1-6.4.
 // ====================================================================================================
-constexpr int kStages64 = 4;      // K and V tiles in flight (16 KB each at D = 64: shared memory has room, and a tile
-                                  // requested only one slot ahead does not always arrive within that slot)
+constexpr int kThreads64 = 640;   // 4 control warps, 4 softmax warpgroups
+constexpr int kStages64 = 3;      // K and V tiles in flight (16 KB each)
 enum BarrierIndex64 {
   k6QFull = 0,
   k6KFirst,
   k6Full0,                                       // [kStages64] V(e) and K(e + 1) have landed (index e % kStages64)
   k6DoneA0 = k6Full0 + kStages64,                // [kStages64] tile A's issuer has finished all its MMAs of slot e
   k6DoneB0 = k6DoneA0 + kStages64,               // [kStages64] the same for tile B
-  k6SFullA = k6DoneB0 + kStages64, k6SFullB,
-  k6SFreeA, k6SFreeB,            // the softmax warpgroup has read S_X into registers (128 arrivals)
-  k6PLoA, k6PHiA, k6PLoB, k6PHiB,
-  k6OFinalA, k6OFinalB,
-  k6NumBarriers
+  k6SFull = k6DoneB0 + kStages64,                // [4] scores of a chain are ready
+  k6OFinal = k6SFull + 4,                        // [2] all products of a query tile are done
+  k6P = k6OFinal + 2,                            // [4] P of a chain has been stored (128 arrivals)
+  k6NumBarriers = k6P + 4
 };
 
 struct __align__(8) Control64 {
@@ -490,8 +485,12 @@ struct __align__(8) Control64 {
   int abort_flag;
 };
 
+// per query tile: 64 accumulator columns, reference and sum of the second chain's rows
+constexpr int kMergeFloats64 = 66 * kTile;
+
 constexpr size_t smem_bytes_d64() {
-  return static_cast<size_t>(2 + 2 * kStages64) * kTile * 64 * 2 + 1024 + sizeof(Control64);
+  return static_cast<size_t>(2 + 2 * kStages64) * kTile * 64 * 2 + 2 * kMergeFloats64 * sizeof(float) + 1024 +
+         sizeof(Control64);
 }
 
 // Maximum of 64 values: eight independent chains of three-input max.
@@ -508,14 +507,14 @@ __device__ __forceinline__ float row_max64(const float* v) {
   return fmaxf(ptx::max3(a[0], a[1], a[2]), ptx::max3(ptx::max3(a[3], a[4], a[5]), a[6], a[7]));
 }
 
-// P = exp2(S * scale - ref) for 64 columns of one row: pk[32] = 16-bit pairs; the row sum goes into the packed sums.
-template <bool kBF16>
-__device__ __forceinline__ void exp_half(const float* v, float scale_log2, float ref, uint32_t* pk, uint64_t& sum2a,
-                                         uint64_t& sum2b) {
+// P = exp2(S * scale - ref) for 2 * kPairs columns of one row: pk = 16-bit pairs; the row sum goes into the packed sums.
+template <bool kBF16, int kPairs>
+__device__ __forceinline__ void exp_pairs(const float* v, float scale_log2, float ref, uint32_t* pk, uint64_t& sum2a,
+                                          uint64_t& sum2b) {
   const uint64_t scale2 = ptx::pack_f32x2(scale_log2, scale_log2);
   const uint64_t nref2 = ptx::pack_f32x2(-ref, -ref);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
+  for (int i = 0; i < kPairs; ++i) {
     const uint64_t x2 = ptx::fma_f32x2(ptx::pack_f32x2(v[2 * i], v[2 * i + 1]), scale2, nref2);
     float x0, x1;
     ptx::unpack_f32x2(x2, x0, x1);
@@ -527,7 +526,7 @@ __device__ __forceinline__ void exp_half(const float* v, float scale_log2, float
 }
 
 template <bool kBF16>
-__global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
+__global__ void __launch_bounds__(kThreads64, 1) sparse_attn_fwd_d64_kernel(
     const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
     const __grid_constant__ CUtensorMap tm_v, const int32_t* __restrict__ counts,
     const int32_t* __restrict__ entries, const int32_t* __restrict__ order, int Hm, int ntk, int N, float scale_log2,
@@ -535,12 +534,13 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
     int32_t* __restrict__ status, const __grid_constant__ OutScatter scatter) {
   constexpr int D = 64;
   constexpr int kTileBytes = kTile * D * 2;       // one Q, K or V tile: 128 rows x 128 bytes
-  constexpr uint32_t kIdescQK = ptx::idesc_f16(128, 128, kBF16, false);
+  constexpr uint32_t kIdescQK = ptx::idesc_f16(128, 64, kBF16, false);
   constexpr uint32_t kIdescPV = ptx::idesc_f16(128, D, kBF16, true);
 
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Control64* ctl = reinterpret_cast<Control64*>(smem + (2 + 2 * kStages64) * kTileBytes);
+  float* merge = reinterpret_cast<float*>(smem + (2 + 2 * kStages64) * kTileBytes);
+  Control64* ctl = reinterpret_cast<Control64*>(merge + 2 * kMergeFloats64);
   const uint32_t sQ = ptx::smem_u32(smem);
   const uint32_t sK = sQ + 2 * kTileBytes;
   const uint32_t sV = sK + kStages64 * kTileBytes;
@@ -561,11 +561,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
   const int32_t* ent = entries + (static_cast<int64_t>(mh) * npairs + pair) * ntk;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < k6NumBarriers; ++i) {
-      uint32_t c = 1;
-      if (i >= k6SFreeA && i <= k6PHiB) c = 128;
-      ptx::mbar_init(bar(i), c);
-    }
+    for (int i = 0; i < k6NumBarriers; ++i) ptx::mbar_init(bar(i), i >= k6P ? 128u : 1u);
     ctl->abort_flag = 0;
     ptx::fence_barrier_init();
     ptx::prefetch_tensormap(&tm_q);
@@ -588,8 +584,9 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
     return static_cast<uint32_t>((((j + kStages64) % kStages64 == kStages64 - 1) ? (j + 1) / kStages64 : j / kStages64) & 1);
   };
 
+  // 640 threads start with 96 registers each, 61,440 in all; of these 128 x 40 + 512 x 104 = 58,368 are kept.
   if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       if (ptx::elect_one()) {
@@ -634,80 +631,71 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
         const uint64_t dqx = ptx::smem_desc_sw128(sQ + x * kTileBytes, 16, 1024);
         const uint64_t dk0 = ptx::smem_desc_sw128(sK, 16, 1024);
         const uint64_t dv0 = ptx::smem_desc_sw128(sV, kTileBytes, 1024);
-        const uint32_t tSx = tmem + x * 128, tOx = tmem + 256 + x * D, tPx = tmem + 384 + x * 64;
         auto advance = [](uint64_t desc, uint32_t bytes) -> uint64_t {
           return (desc & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(desc) + (bytes >> 4));
         };
-        auto issue_qk = [&](int s) {          // s: K stage
-          const uint64_t b0 = advance(dk0, static_cast<uint32_t>(s) * kTileBytes);
+        // the 64-key halves of an entry that the tile keeps in either half of its rows
+        auto halves = [&](int e) -> uint32_t {
+          const uint32_t f = static_cast<uint32_t>(ent[e]) >> (4 * x);
+          return (f | (f >> 2)) & 3u;
+        };
+        auto issue_qk = [&](int h, int s) {   // s: K stage
+          const uint64_t b0 = advance(dk0, static_cast<uint32_t>(s) * kTileBytes + h * (kTileBytes / 2));
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk)
-            ptx::mma_ss(tSx, advance(dqx, kk * 32), advance(b0, kk * 32), kIdescQK, kk > 0 ? 1u : 0u);
-          ptx::tc_commit(bar(k6SFullA + x));
-        };
-        auto issue_pv_half = [&](int s, int half, uint32_t acc) {   // s: V stage
-          const uint64_t b0 = advance(dv0, static_cast<uint32_t>(s) * kTileBytes);
-#pragma unroll
-          for (int kq = 0; kq < 4; ++kq) {
-            const int kk = half * 4 + kq;
-            ptx::mma_ts(tOx, tPx + kk * 8, advance(b0, kk * 2048), kIdescPV, (acc || kq > 0) ? 1u : 0u);
-          }
+            ptx::mma_ss(tmem + (2 * x + h) * 64, advance(dqx, kk * 32), advance(b0, kk * 32), kIdescQK, kk > 0 ? 1u : 0u);
+          ptx::tc_commit(bar(k6SFull + 2 * x + h));
         };
         bool ok = ptx::mbar_wait(bar(k6QFull), 0, abort_flag);
         if (!ok) report(status, 2, 1 + x, -1);
-        // flags of entry e, e + 1 and e + 2: each is loaded two slots before the issuer needs it (a load issued
+        // halves of entry e, e + 1 and e + 2: each is loaded two slots before the issuer needs it (a load issued
         // where its value is used would put a trip to the L2 on the issuing thread's path every slot)
-        int sub = (cnt > 0) ? ((ent[0] >> (4 * x)) & 0xf) : 0;
-        int subn = (cnt > 1) ? ((ent[1] >> (4 * x)) & 0xf) : 0;
-        int n_qk = 0;                       // Q K^T products issued so far for this tile
+        uint32_t sub = (cnt > 0) ? halves(0) : 0u, subn = (cnt > 1) ? halves(1) : 0u;
         if (ok && cnt > 0) {
           ok = ptx::mbar_wait(bar(k6KFirst), 0, abort_flag);
           if (!ok) report(status, 2, 1 + x, 0);
           if (ok) {
             ptx::tc_fence_after();
-            if (sub) { issue_qk(0); ++n_qk; }
+            if (sub & 1u) issue_qk(0, 0);
+            if (sub & 2u) issue_qk(1, 0);
             ptx::tc_commit(bar(k6DoneA0 + kStages64 * x + kStages64 - 1));   // "slot -1": K stage 0 is free again
           }
         }
-        uint32_t par_p = 0, acc = 0;
+        uint32_t par_p = 0, acc = 0;          // a bit per chain
         for (int e = 0; e < cnt && ok; ++e) {
           const int s = e % kStages64;
-          const int subnn = (e + 2 < cnt) ? ((ent[e + 2] >> (4 * x)) & 0xf) : 0;   // first used in the next slot
+          const uint32_t subnn = (e + 2 < cnt) ? halves(e + 2) : 0u;   // first used in the next slot
           ok = ptx::mbar_wait(bar(k6Full0 + s), (e / kStages64) & 1, abort_flag);
           if (!ok) { report(status, 2, 1 + x, e); break; }
-          if (subn) {
-            // S_x is free once the softmax has read the scores of the tile's previous entry
-            if (n_qk > 0) {
-              ok = ptx::mbar_wait(bar(k6SFreeA + x), static_cast<uint32_t>((n_qk - 1) & 1), abort_flag);
-              if (!ok) { report(status, 6, 1 + x, e); break; }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if ((sub >> h) & 1u) {
+              ok = ptx::mbar_wait(bar(k6P + 2 * x + h), (par_p >> h) & 1u, abort_flag);
+              if (!ok) { report(status, 3, 1 + x, e); break; }
+              ptx::tc_fence_after();
+              const uint64_t b0 = advance(dv0, static_cast<uint32_t>(s) * kTileBytes + h * (kTileBytes / 2));
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk)
+                ptx::mma_ts(tmem + 256 + (2 * x + h) * 64, tmem + (2 * x + h) * 64 + kk * 8, advance(b0, kk * 2048), kIdescPV,
+                            (((acc >> h) & 1u) || kk > 0) ? 1u : 0u);
+              par_p ^= 1u << h;
+              acc |= 1u << h;
             }
-            ptx::tc_fence_after();
-            issue_qk((e + 1) % kStages64);
-            ++n_qk;
+            if ((subn >> h) & 1u) issue_qk(h, (e + 1) % kStages64);
           }
-          if (sub) {
-            ok = ptx::mbar_wait(bar(k6PLoA + 2 * x), par_p, abort_flag);
-            if (!ok) { report(status, 3, 1 + x, e); break; }
-            ptx::tc_fence_after();
-            issue_pv_half(s, 0, acc);
-            ok = ptx::mbar_wait(bar(k6PHiA + 2 * x), par_p, abort_flag);
-            if (!ok) { report(status, 3, 1 + x, e); break; }
-            ptx::tc_fence_after();
-            issue_pv_half(s, 1, 1u);
-            par_p ^= 1;
-            acc = 1u;
-          }
+          if (!ok) break;
           ptx::tc_commit(bar(k6DoneA0 + kStages64 * x + s));  // this tile's MMAs of slot e are done
           sub = subn;
           subn = subnn;
         }
-        ptx::tc_commit(bar(k6OFinalA + x));
+        ptx::tc_commit(bar(k6OFinal + x));
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     // ------------------------------------------------------------------ softmax + epilogue
-    const int x = (warp - 4) / 4;                 // 0: tile A, 1: tile B
+    const int chain = (warp - 4) / 4;             // 2 * query tile + key half
+    const int x = chain >> 1, h = chain & 1;
     const int wq = warp % 4;                      // tensor-memory lane quarter of this warp
     const int r = wq * 32 + lane;                 // row inside the tile
     const int tile = 2 * pair + x;
@@ -715,10 +703,10 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
     const int kvl = (grow < q_split) ? kvl_lo : kvl_hi;
     const int kvl_min = min(kvl_lo, kvl_hi);
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-    const uint32_t tS = tmem + lane_base + x * 128;
-    const uint32_t tO = tmem + lane_base + 256 + x * D;
-    const uint32_t tP = tmem + lane_base + 384 + x * 64;
-    const int rh = r >> 6;                        // row half of the tile: the same for the whole warp
+    const uint32_t tS = tmem + lane_base + chain * 64;
+    const uint32_t tO = tmem + lane_base + 256 + chain * 64;
+    const int bit_mine = 4 * x + 2 * (r >> 6) + h;     // flag of this row half (the same for the whole warp)
+    const int bits_both = 0x5 << (4 * x + h);          // flags of this key half, both row halves
 
     float m = -INFINITY, l = 0.f;
     uint32_t par_s = 0;
@@ -728,92 +716,101 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
     for (int e = 0; e < cnt; ++e) {
       const int en = en_next;
       en_next = (e + 1 < cnt) ? ent[e + 1] : 0;   // in flight while this entry is processed
-      const int sub = (en >> (4 * x)) & 0xf;
-      if (!sub) continue;
-      const int col0 = (en >> 8) * kTile;
-      ok = ptx::mbar_wait(bar(k6SFullA + x), par_s, abort_flag);
+      if (!(en & bits_both)) continue;
+      ok = ptx::mbar_wait(bar(k6SFull + chain), par_s, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok) { if (lane == 0) report(status, 4, 2 + x, e); break; }
+      if (!ok) { if (lane == 0) report(status, 4, 2 + chain, e); break; }
       par_s ^= 1;
       ptx::tc_fence_after();
-      // per 64-key half (flags are the same for every thread of the warp): keep = the rows of this warp keep it
-      const bool keep[2] = {((sub >> (2 * rh)) & 1) != 0, ((sub >> (2 * rh + 1)) & 1) != 0};
-      const bool edge = col0 + kTile > kvl_min;   // the tile reaches past the valid keys of some row
-      float v[kTile];
+      if ((en >> bit_mine) & 1) {
+        float v[64];
+        ptx::tmem_ld32(tS, reinterpret_cast<uint32_t*>(v));
+        ptx::tmem_ld32(tS + 32, reinterpret_cast<uint32_t*>(v) + 32);
+        ptx::tmem_ld_wait();
+        const int col0 = (en >> 8) * kTile + h * 64;
+        if (col0 + 64 > kvl_min) {                // the half reaches past the valid keys of some row
+          const int lim = kvl - col0;             // columns >= lim are beyond the valid keys of this row
 #pragma unroll
-      for (int half = 0; half < 2; ++half)
-        if (keep[half]) {
-          ptx::tmem_ld32(tS + half * 64, reinterpret_cast<uint32_t*>(v) + half * 64);
-          ptx::tmem_ld32(tS + half * 64 + 32, reinterpret_cast<uint32_t*>(v) + half * 64 + 32);
+          for (int c = 0; c < 64; ++c) v[c] = (c < lim) ? v[c] : -INFINITY;
         }
-      ptx::tmem_ld_wait();
-      ptx::tc_fence_before();
-      ptx::mbar_arrive(bar(k6SFreeA + x));        // the next Q K^T of this tile may overwrite S
-      if (edge) {
-        const int lim = kvl - col0;               // columns >= lim are beyond the valid keys of this row
-#pragma unroll
-        for (int c = 0; c < kTile; ++c)
-          if (keep[c / 64]) v[c] = (c < lim) ? v[c] : -INFINITY;
-      }
-      float mx = -INFINITY;
-#pragma unroll
-      for (int half = 0; half < 2; ++half)
-        if (keep[half]) mx = fmaxf(mx, row_max64(v + half * 64));
-      const float m_new = fmaxf(m, mx * scale_log2);
-      // this tile's products of the previous slot have completed: P_x may be overwritten and O_x may be rescaled
-      if (e > 0) {
-        ok = ptx::mbar_wait(bar(k6DoneA0 + kStages64 * x + done_index(e - 1)), done_parity(e - 1), abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) { if (lane == 0) report(status, 7, 2 + x, e); break; }
-        ptx::tc_fence_after();
-      }
-      if (done == 0) {
-        m = m_new;
-      } else if (__any_sync(0xffffffffu, m_new > m + kRescaleThreshold)) {
+        const float m_new = fmaxf(m, row_max64(v) * scale_log2);
+        // A new reference rescales O; that is done below, before P is handed over, so that the exponentials follow the
+        // row maximum in one piece of straight code.
+        const bool rescale = done > 0 && __any_sync(0xffffffffu, m_new > m + kRescaleThreshold);
         const float alpha = (m == -INFINITY) ? 0.f : ptx::ex2(m - m_new);
-        l *= alpha;
-        m = m_new;
+        if (rescale) l *= alpha;
+        if (rescale || done == 0) m = m_new;
+        const float ref = (m == -INFINITY) ? 0.f : m;
+        uint64_t sum2a = 0, sum2b = 0;    // bit pattern of (0.f, 0.f)
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-          float o[32];
-          ptx::tmem_ld32(tO + c * 32, reinterpret_cast<uint32_t*>(o));
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] *= alpha;
-          ptx::tmem_st32(tO + c * 32, reinterpret_cast<const uint32_t*>(o));
+        for (int part = 0; part < 2; ++part) {
+          uint32_t pk[16];
+          exp_pairs<kBF16, 16>(v + 32 * part, scale_log2, ref, pk, sum2a, sum2b);
+          ptx::tmem_st16(tS + 16 * part, pk);
         }
-      }
-      const float ref = (m == -INFINITY) ? 0.f : m;
-      uint64_t sum2a = 0, sum2b = 0;    // bit pattern of (0.f, 0.f)
+        float s0, s1, s2, s3;
+        ptx::unpack_f32x2(sum2a, s0, s1);
+        ptx::unpack_f32x2(sum2b, s2, s3);
+        l += (s0 + s1) + (s2 + s3);
+        if (rescale) {
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t pk[32];
-        if (keep[half]) {
-          exp_half<kBF16>(v + half * 64, scale_log2, ref, pk, sum2a, sum2b);
-        } else {
+          for (int c = 0; c < D / 16; ++c) {
+            float o[16];
+            ptx::tmem_ld16(tO + c * 16, reinterpret_cast<uint32_t*>(o));
+            ptx::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) pk[i] = 0u;   // a half this row half does not keep: no exponentials at all
+            for (int i = 0; i < 16; ++i) o[i] *= alpha;
+            ptx::tmem_st16(tO + c * 16, reinterpret_cast<const uint32_t*>(o));
+          }
         }
-        ptx::tmem_st32(tP + half * 32, pk);
-        ptx::tmem_st_wait();
-        ptx::tc_fence_before();
-        ptx::mbar_arrive(bar(k6PLoA + 2 * x + half));
+      } else {
+        uint32_t pk[16];                          // a half this row half does not keep: no exponentials at all
+#pragma unroll
+        for (int i = 0; i < 16; ++i) pk[i] = 0u;
+        ptx::tmem_st16(tS, pk);
+        ptx::tmem_st16(tS + 16, pk);
       }
-      float s0, s1, s2, s3;
-      ptx::unpack_f32x2(sum2a, s0, s1);
-      ptx::unpack_f32x2(sum2b, s2, s3);
-      l += (s0 + s1) + (s2 + s3);
+      ptx::tmem_st_wait();
+      ptx::tc_fence_before();
+      ptx::mbar_arrive(bar(k6P + chain));
       ++done;
     }
 
     if (ok) {
-      ok = ptx::mbar_wait(bar(k6OFinalA + x), 0, abort_flag);
+      ok = ptx::mbar_wait(bar(k6OFinal + x), 0, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok && lane == 0) report(status, 5, 2 + x, -1);
+      if (!ok && lane == 0) report(status, 5, 2 + chain, -1);
     }
-    if (ok && tile < ntq) {
-      ptx::tc_fence_after();
-      const float inv = (done > 0 && l > 0.f) ? 1.f / l : 0.f;
+    ptx::tc_fence_after();
+    // The second chain hands its rows to the first through shared memory, which puts the two together and stores them.
+    float* mg = merge + x * kMergeFloats64;
+    if (h == 1) {
+#pragma unroll
+      for (int c = 0; c < D / 16; ++c) {
+        float o[16];
+        if (done > 0 && ok) {
+          ptx::tmem_ld16(tO + c * 16, reinterpret_cast<uint32_t*>(o));
+          ptx::tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[i] = 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) mg[(c * 16 + i) * kTile + r] = o[i];
+      }
+      mg[64 * kTile + r] = m;
+      mg[65 * kTile + r] = l;
+    }
+    if (x == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+    else asm volatile("bar.sync 2, 256;" ::: "memory");
+    if (h == 0 && ok && tile < ntq) {
+      const float m1 = mg[64 * kTile + r], l1 = mg[65 * kTile + r];
+      const float mm = fmaxf(m, m1);
+      const float w0 = (m == -INFINITY) ? 0.f : ptx::ex2(m - mm);
+      const float w1 = (m1 == -INFINITY) ? 0.f : ptx::ex2(m1 - mm);
+      const float lt = l * w0 + l1 * w1;
+      const float inv = lt > 0.f ? 1.f / lt : 0.f;
+      const float f0 = w0 * inv, f1 = w1 * inv;
       uint4* dst;
       if (scatter.n_peers > 0) {
         const int pr = min(grow / scatter.rows_per_peer, scatter.n_peers - 1);
@@ -824,30 +821,31 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_d64_kernel(
         dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(out_raw) + (static_cast<int64_t>(bh) * N + grow) * D * 2);
       }
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        float o[32];
+      for (int c = 0; c < D / 16; ++c) {
+        float o[16];
         if (done > 0) {
-          ptx::tmem_ld32(tO + c * 32, reinterpret_cast<uint32_t*>(o));
+          ptx::tmem_ld16(tO + c * 16, reinterpret_cast<uint32_t*>(o));
           ptx::tmem_ld_wait();
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0.f;
+          for (int i = 0; i < 16; ++i) o[i] = 0.f;
         }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[i] = o[i] * f0 + mg[(c * 16 + i) * kTile + r] * f1;
         if (grow < N) {
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
+          for (int q4 = 0; q4 < 2; ++q4) {
             uint4 w;
-            w.x = pack2<kBF16>(o[q4 * 8 + 0] * inv, o[q4 * 8 + 1] * inv);
-            w.y = pack2<kBF16>(o[q4 * 8 + 2] * inv, o[q4 * 8 + 3] * inv);
-            w.z = pack2<kBF16>(o[q4 * 8 + 4] * inv, o[q4 * 8 + 5] * inv);
-            w.w = pack2<kBF16>(o[q4 * 8 + 6] * inv, o[q4 * 8 + 7] * inv);
-            dst[c * 4 + q4] = w;
+            w.x = pack2<kBF16>(o[q4 * 8 + 0], o[q4 * 8 + 1]);
+            w.y = pack2<kBF16>(o[q4 * 8 + 2], o[q4 * 8 + 3]);
+            w.z = pack2<kBF16>(o[q4 * 8 + 4], o[q4 * 8 + 5]);
+            w.w = pack2<kBF16>(o[q4 * 8 + 6], o[q4 * 8 + 7]);
+            dst[c * 2 + q4] = w;
           }
         }
       }
       if (lse != nullptr && grow < N) {
-        lse[static_cast<int64_t>(bh) * N + grow] =
-            (done > 0 && l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+        lse[static_cast<int64_t>(bh) * N + grow] = lt > 0.f ? (mm + log2f(lt)) * 0.6931471805599453f : -INFINITY;
       }
     }
   }
@@ -874,8 +872,8 @@ int launch_d64(const void* q, const void* k, const void* v, int dtype, int BH, i
   const size_t smem = smem_bytes_d64();
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  kernel<<<dim3(npairs * Hm, BH / Hm), kThreads, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N, scale_log2,
-                                                            q_split, kvl_lo, kvl_hi, out, lse, status, scatter);
+  kernel<<<dim3(npairs * Hm, BH / Hm), kThreads64, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N, scale_log2,
+                                                              q_split, kvl_lo, kvl_hi, out, lse, status, scatter);
   MODDIT_CHECK_LAUNCH("sparse_attn_fwd_d64_kernel");
   return MODDIT_OK;
 }
