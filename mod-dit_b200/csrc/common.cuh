@@ -52,4 +52,11 @@ int ensure_dynamic_smem(const void* kernel, size_t bytes);
 // Number of SMs of the current device.
 int sm_count(int* sms);
 
+// Stages of a prediction in fewer launches than their entry points make (moddit_predict_lines; arguments as there, the
+// workspaces are those of moddit_pooled_map_ws and moddit_solve).
+int pooled_map_of_blocks(const void* q, const void* k, int dtype, int BH, int N, int D, int block_size, int first, int n,
+                         float scale, void* map_f16, void* workspace, cudaStream_t st);
+int solve_features(const float* mts, const void* factor, bool small, int H, int n, float threshold, float* d, float* c,
+                   float* b_d, int32_t* modes, void* workspace, size_t workspace_bytes, void* stream);
+
 }  // namespace moddit

@@ -238,9 +238,33 @@ __global__ void __launch_bounds__(kSmallFactorThreads) solve_small_factor_kernel
   }
 }
 
+// Where a solution goes: unknown i of head h to X (H, 3n), or, in the form in which the steps after it read it (d non-null),
+// diagonals, halved columns, block coefficient and the head's mode from the latter.
+struct SolutionOut {
+  float* X;
+  float* d;
+  float* c;
+  float* b_d;
+  int32_t* modes;
+  float threshold;
+};
+__device__ __forceinline__ void put_unknown(const SolutionOut& o, int h, int i, int n, float x) {
+  const int nd = 2 * n - 1;
+  if (o.d == nullptr) {
+    o.X[static_cast<int64_t>(h) * 3 * n + i] = x;
+  } else if (i < nd) {
+    o.d[static_cast<int64_t>(h) * nd + i] = x;
+  } else if (i < nd + n) {
+    o.c[static_cast<int64_t>(h) * n + (i - nd)] = x / 2.f;
+  } else {
+    o.b_d[h] = x;
+    if (o.modes != nullptr) o.modes[h] = (x <= o.threshold) ? MODDIT_MODE_BLOCK_DIAGONAL : MODDIT_MODE_SPARSE;
+  }
+}
+
 __global__ void __launch_bounds__(kSmallThreads) solve_small_kernel(const float* __restrict__ mts,
                                                                     const float* __restrict__ inv, int H, int n,
-                                                                    float* __restrict__ X) {
+                                                                    const __grid_constant__ SolutionOut out) {
   const int F = 3 * n;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int i = blockIdx.y * (kSmallThreads / 32) + warp;
@@ -261,7 +285,7 @@ __global__ void __launch_bounds__(kSmallThreads) solve_small_kernel(const float*
   for (int hh = 0; hh < kSmallHeads; ++hh) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc[hh] += __shfl_xor_sync(0xffffffffu, acc[hh], o);
-    if (lane == 0 && h0 + hh < H) X[static_cast<int64_t>(h0 + hh) * F + i] = static_cast<float>(acc[hh]);
+    if (lane == 0 && h0 + hh < H) put_unknown(out, h0 + hh, i, n, static_cast<float>(acc[hh]));
   }
 }
 
@@ -458,7 +482,7 @@ __global__ void __launch_bounds__(kSolveThreads) solve_back_kernel(const float* 
                                                                    const double* __restrict__ w,
                                                                    const double* __restrict__ wb,
                                                                    const double* __restrict__ y, int n,
-                                                                   float* __restrict__ X) {
+                                                                   const __grid_constant__ SolutionOut out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* pc = reinterpret_cast<double*>(smem_raw);  // [n] inclusive prefix of c
   double* carry = pc + n;                            // [kSolveThreads]
@@ -467,7 +491,6 @@ __global__ void __launch_bounds__(kSolveThreads) solve_back_kernel(const float* 
   const int nd = 2 * n - 1;
   const int m = n + 1;
   const float* r = mts + static_cast<int64_t>(h) * 3 * n;
-  float* xh = X + static_cast<int64_t>(h) * 3 * n;
   auto y_at = [&](int j) {          // sum of the gemv slices, always in the same order
     double acc = 0.0;
     for (int sl = 0; sl < kGemvSplit; ++sl) acc += y[(static_cast<int64_t>(sl) * H + h) * m + j];
@@ -476,10 +499,10 @@ __global__ void __launch_bounds__(kSolveThreads) solve_back_kernel(const float* 
   for (int j = threadIdx.x; j < n; j += kSolveThreads) {
     const double yj = y_at(j);
     pc[j] = yj;
-    xh[nd + j] = static_cast<float>(yj);
+    put_unknown(out, h, nd + j, n, static_cast<float>(yj));
   }
   const double e = y_at(n);
-  if (threadIdx.x == 0) xh[nd + n] = static_cast<float>(e);
+  if (threadIdx.x == 0) put_unknown(out, h, nd + n, n, static_cast<float>(e));
   __syncthreads();
   block_scan_inclusive(pc, n, carry);
   const double total = pc[n - 1];
@@ -487,7 +510,7 @@ __global__ void __launch_bounds__(kSolveThreads) solve_back_kernel(const float* 
     const int o = oi - (n - 1);
     // (A c)[o] = sum_{j>=o} c_j for o >= 0 ; sum_{j<n+o} c_j for o < 0
     const double ac = (o >= 0) ? (total - (o > 0 ? pc[o - 1] : 0.0)) : pc[n + o - 1];
-    xh[oi] = static_cast<float>(w[oi] * (static_cast<double>(r[oi]) - ac) - wb[oi] * e);
+    put_unknown(out, h, oi, n, static_cast<float>(w[oi] * (static_cast<double>(r[oi]) - ac) - wb[oi] * e));
   }
 }
 
@@ -625,17 +648,8 @@ __global__ void __launch_bounds__(256) split_solution_kernel(const float* __rest
                                                              float* __restrict__ d, float* __restrict__ c,
                                                              float* __restrict__ b_d, int32_t* __restrict__ modes) {
   const int h = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x;
-  const int nd = 2 * n - 1;
   if (i >= 3 * n) return;
-  const float x = X[static_cast<int64_t>(h) * 3 * n + i];
-  if (i < nd) {
-    d[static_cast<int64_t>(h) * nd + i] = x;
-  } else if (i < nd + n) {
-    c[static_cast<int64_t>(h) * n + (i - nd)] = x / 2.f;
-  } else {
-    b_d[h] = x;
-    if (modes != nullptr) modes[h] = (x <= threshold) ? MODDIT_MODE_BLOCK_DIAGONAL : MODDIT_MODE_SPARSE;
-  }
+  put_unknown({nullptr, d, c, b_d, modes, threshold}, h, i, n, X[static_cast<int64_t>(h) * 3 * n + i]);
 }
 }  // namespace
 }  // namespace moddit
@@ -733,12 +747,9 @@ extern "C" size_t moddit_solve_workspace_bytes(int H, int n) {
   return sizeof(double) * (1 + kGemvSplit) * static_cast<size_t>(H) * (static_cast<size_t>(n) + 1);
 }
 
-extern "C" int moddit_solve(const float* mts, const void* factor, int H, int n, int blocks_per_frame,
-                            double regularization, float* X, void* workspace, size_t workspace_bytes, void* stream) {
-  clear_error();
-  (void)blocks_per_frame;
-  (void)regularization;
-  MODDIT_CHECK_ARG(mts && factor && X, "solve: null pointer");
+static int solve_into(const SolutionOut& out, const float* mts, const void* factor, int H, int n, void* workspace,
+                      size_t workspace_bytes, void* stream) {
+  MODDIT_CHECK_ARG(mts && factor && (out.X || (out.d && out.c && out.b_d)), "solve: null pointer");
   MODDIT_CHECK_ARG(H > 0 && H <= 65535, "solve: H=%d outside [1, 65535]", H);
   if (int rc = check_n("solve", n)) return rc;
   if (!workspace || workspace_bytes < moddit_solve_workspace_bytes(H, n))
@@ -762,9 +773,17 @@ extern "C" int moddit_solve(const float* mts, const void* factor, int H, int n, 
   solve_gemv_kernel<<<dim3(ceil_div(m, 128), ceil_div(H, kGemvHeads), kGemvSplit), 128,
                       sizeof(double) * kGemvHeads * ceil_div(m, kGemvSplit), st>>>(Sinv, g, m, H, y);
   MODDIT_CHECK_LAUNCH("solve_gemv_kernel");
-  solve_back_kernel<<<H, kSolveThreads, sm_back, st>>>(mts, w, wb, y, n, X);
+  solve_back_kernel<<<H, kSolveThreads, sm_back, st>>>(mts, w, wb, y, n, out);
   MODDIT_CHECK_LAUNCH("solve_back_kernel");
   return MODDIT_OK;
+}
+
+extern "C" int moddit_solve(const float* mts, const void* factor, int H, int n, int blocks_per_frame,
+                            double regularization, float* X, void* workspace, size_t workspace_bytes, void* stream) {
+  clear_error();
+  (void)blocks_per_frame;
+  (void)regularization;
+  return solve_into({X, nullptr, nullptr, nullptr, nullptr, 0.f}, mts, factor, H, n, workspace, workspace_bytes, stream);
 }
 
 extern "C" int moddit_solve_small_max_n(void) { return kSmallMaxF / 3; }
@@ -798,15 +817,26 @@ extern "C" int moddit_solve_small_prepare(int n, int blocks_per_frame, float reg
   return MODDIT_OK;
 }
 
-extern "C" int moddit_solve_small(const float* mts, const float* factor, int H, int n, float* X, void* stream) {
-  clear_error();
-  MODDIT_CHECK_ARG(mts && factor && X, "solve_small: null pointer");
+static int solve_small_into(const SolutionOut& out, const float* mts, const float* factor, int H, int n, void* stream) {
+  MODDIT_CHECK_ARG(mts && factor && (out.X || (out.d && out.c && out.b_d)), "solve_small: null pointer");
   MODDIT_CHECK_ARG(H > 0 && H <= 65535 * (kSmallThreads / 32), "solve_small: H=%d out of range", H);
   if (int rc = check_small("solve_small", n)) return rc;
   if (int rc = require_sm100()) return rc;
   const int F = 3 * n;
   solve_small_kernel<<<dim3(ceil_div(H, kSmallHeads), ceil_div(F, kSmallThreads / 32)), kSmallThreads, 0, as_stream(stream)>>>(
-      mts, factor, H, n, X);
+      mts, factor, H, n, out);
   MODDIT_CHECK_LAUNCH("solve_small_kernel");
   return MODDIT_OK;
+}
+
+extern "C" int moddit_solve_small(const float* mts, const float* factor, int H, int n, float* X, void* stream) {
+  clear_error();
+  return solve_small_into({X, nullptr, nullptr, nullptr, nullptr, 0.f}, mts, factor, H, n, stream);
+}
+
+int moddit::solve_features(const float* mts, const void* factor, bool small, int H, int n, float threshold, float* d, float* c,
+                           float* b_d, int32_t* modes, void* workspace, size_t workspace_bytes, void* stream) {
+  const SolutionOut out = {nullptr, d, c, b_d, modes, threshold};
+  return small ? solve_small_into(out, mts, static_cast<const float*>(factor), H, n, stream)
+               : solve_into(out, mts, factor, H, n, workspace, workspace_bytes, stream);
 }

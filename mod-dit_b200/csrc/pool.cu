@@ -59,19 +59,32 @@ struct PoolShard {
   int block_base;
 };
 
+// The form in which a prediction pools (kSplit): query (blockIdx.z 0) and key (1) in one launch, blocks first, first + 1, ...
+// only, and the means leave as the two bfloat16 terms that the logits kernel reads ((BH, n, 2, D), query means times
+// `scale`) - what pool_blocks of either tensor and split_means_kernel give, without the float32 means in between.
+struct PoolSplit {
+  const void* k;
+  __nv_bfloat16* qs;
+  __nv_bfloat16* ks;
+  float scale;
+  int first;
+};
+
 // D is 64 or 128: D/8 threads cover one row with one 16-byte load each.
-template <typename T, int D, bool kShard>
+template <typename T, int D, bool kShard, bool kSplit = false>
 __global__ void __launch_bounds__(kPoolThreads) pool_blocks_kernel(const T* __restrict__ x, int N, int bs,
                                                                    float* __restrict__ out,
-                                                                   const __grid_constant__ PoolShard shard) {
+                                                                   const __grid_constant__ PoolShard shard,
+                                                                   const __grid_constant__ PoolSplit split) {
   constexpr int kTpr = D / 8;                   // threads per row
   constexpr int kRpp = kPoolThreads / kTpr;     // rows per pass
   __shared__ float red[kRpp][D];
 
-  const int blk = blockIdx.x;
+  const int blk = (kSplit ? split.first : 0) + blockIdx.x;
   const int bh = blockIdx.y;
   const int nb = gridDim.x;
   const int row0 = blk * bs;
+  if (kSplit && blockIdx.z != 0) x = static_cast<const T*>(split.k);
   const int halo_rows = kShard ? shard.halo_rows : 0;
   const int rows = min(bs, halo_rows + N - row0);
   const int cg = threadIdx.x % kTpr;
@@ -113,6 +126,15 @@ __global__ void __launch_bounds__(kPoolThreads) pool_blocks_kernel(const T* __re
     float s = 0.f;
 #pragma unroll 8
     for (int g = 0; g < kRpp; ++g) s += red[g][threadIdx.x];
+    if constexpr (kSplit) {
+      float v = s / static_cast<float>(rows);
+      if (blockIdx.z == 0) v *= split.scale;
+      const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+      __nv_bfloat16* dst = (blockIdx.z == 0 ? split.qs : split.ks) + (static_cast<int64_t>(bh) * nb + blockIdx.x) * 2 * D;
+      dst[threadIdx.x] = hi;
+      dst[D + threadIdx.x] = __float2bfloat16_rn(v - __bfloat162float(hi));
+      return;
+    }
     float* dst;
     if constexpr (kShard) {
       const int owner = bh / shard.heads_per_peer;
@@ -199,23 +221,21 @@ __global__ void __launch_bounds__(kPoolThreads) block_similarity_kernel(const T*
   }
 }
 
-template <bool kShard>
+template <bool kShard, bool kSplit = false>
 void launch_pool(const void* x, int dtype, int D, int N, int bs, float* out, const PoolShard& shard, dim3 grid,
-                 cudaStream_t st) {
+                 cudaStream_t st, const PoolSplit& split = {}) {
   if (dtype == MODDIT_BF16) {
+    const __nv_bfloat16* in = static_cast<const __nv_bfloat16*>(x);
     if (D == 64)
-      pool_blocks_kernel<__nv_bfloat16, 64, kShard><<<grid, kPoolThreads, 0, st>>>(
-          static_cast<const __nv_bfloat16*>(x), N, bs, out, shard);
+      pool_blocks_kernel<__nv_bfloat16, 64, kShard, kSplit><<<grid, kPoolThreads, 0, st>>>(in, N, bs, out, shard, split);
     else
-      pool_blocks_kernel<__nv_bfloat16, 128, kShard><<<grid, kPoolThreads, 0, st>>>(
-          static_cast<const __nv_bfloat16*>(x), N, bs, out, shard);
+      pool_blocks_kernel<__nv_bfloat16, 128, kShard, kSplit><<<grid, kPoolThreads, 0, st>>>(in, N, bs, out, shard, split);
   } else {
+    const __half* in = static_cast<const __half*>(x);
     if (D == 64)
-      pool_blocks_kernel<__half, 64, kShard><<<grid, kPoolThreads, 0, st>>>(static_cast<const __half*>(x), N, bs, out,
-                                                                           shard);
+      pool_blocks_kernel<__half, 64, kShard, kSplit><<<grid, kPoolThreads, 0, st>>>(in, N, bs, out, shard, split);
     else
-      pool_blocks_kernel<__half, 128, kShard><<<grid, kPoolThreads, 0, st>>>(static_cast<const __half*>(x), N, bs, out,
-                                                                            shard);
+      pool_blocks_kernel<__half, 128, kShard, kSplit><<<grid, kPoolThreads, 0, st>>>(in, N, bs, out, shard, split);
   }
 }
 
@@ -521,10 +541,7 @@ size_t pooled_map_smem(int D, int n) {
 
 using namespace moddit;
 
-extern "C" int moddit_pool_blocks(const void* x, int dtype, int BH, int N, int D, int block_size, float* out,
-                                  void* stream) {
-  clear_error();
-  MODDIT_CHECK_ARG(x && out, "pool_blocks: null pointer");
+static int check_pool(const void* x, int dtype, int BH, int N, int D, int block_size) {
   MODDIT_CHECK_ARG(BH > 0 && N > 0, "pool_blocks: BH=%d N=%d must be positive", BH, N);
   if (D != 64 && D != 128) return fail(MODDIT_E_UNSUPPORTED, "pool_blocks: head_dim must be 64 or 128, got %d", D);
   if (block_size != 64 && block_size != 128)
@@ -532,7 +549,14 @@ extern "C" int moddit_pool_blocks(const void* x, int dtype, int BH, int N, int D
   if (dtype != MODDIT_BF16 && dtype != MODDIT_FP16) return fail(MODDIT_E_ARG, "pool_blocks: unknown dtype %d", dtype);
   if (!aligned16(x)) return fail(MODDIT_E_ALIGN, "pool_blocks: input must be 16-byte aligned");
   if (BH > 65535) return fail(MODDIT_E_UNSUPPORTED, "pool_blocks: BH=%d exceeds 65535", BH);
-  if (int rc = require_sm100()) return rc;
+  return require_sm100();
+}
+
+extern "C" int moddit_pool_blocks(const void* x, int dtype, int BH, int N, int D, int block_size, float* out,
+                                  void* stream) {
+  clear_error();
+  MODDIT_CHECK_ARG(x && out, "pool_blocks: null pointer");
+  if (int rc = check_pool(x, dtype, BH, N, D, block_size)) return rc;
   const dim3 grid(ceil_div(N, block_size), BH);
   const PoolShard none = {};
   launch_pool<false>(x, dtype, D, N, block_size, out, none, grid, as_stream(stream));
@@ -639,6 +663,20 @@ extern "C" int moddit_pooled_map(const float* qbar, const float* kbar, int BH, i
   return MODDIT_OK;
 }
 
+// logits and rows of the pooled map from means that are split already
+static int map_of_split_means(const __nv_bfloat16* qs, const __nv_bfloat16* ks, int BH, int D, int n, float* lg, void* map_f16,
+                              cudaStream_t st) {
+  const size_t sm = pooled_logits_smem(D);
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(pooled_logits_kernel), sm)) return rc;
+  pooled_logits_kernel<<<dim3(ceil_div(n, kLgCols), ceil_div(n, kLgRows), BH), kMapThreads, sm, st>>>(qs, ks, D, n, lg);
+  MODDIT_CHECK_LAUNCH("pooled_logits_kernel");
+  const int64_t rows = static_cast<int64_t>(BH) * n;
+  pooled_darkness_kernel<<<static_cast<unsigned>((rows + kMapThreads / 32 - 1) / (kMapThreads / 32)), kMapThreads, 0, st>>>(
+      lg, rows, n, static_cast<__half*>(map_f16));
+  MODDIT_CHECK_LAUNCH("pooled_darkness_kernel");
+  return MODDIT_OK;
+}
+
 extern "C" size_t moddit_pooled_map_workspace_bytes(int BH, int n, int D) {
   if (BH <= 0 || n <= 0 || D <= 0) return 0;
   return pooled_ws_logits_bytes(BH, n) + 2 * pooled_ws_split_bytes(BH, n, D);
@@ -662,8 +700,6 @@ extern "C" int moddit_pooled_map_ws(const float* qbar, const float* kbar, int BH
                 "pooled_map_ws: head_dim must be a multiple of 16 (at most 256), inputs and workspace 16-byte aligned");
   if (int rc = require_sm100()) return rc;
   cudaStream_t st = as_stream(stream);
-  const size_t sm = pooled_logits_smem(D);
-  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(pooled_logits_kernel), sm)) return rc;
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   float* lg = reinterpret_cast<float*>(ws);
   __nv_bfloat16* qs = reinterpret_cast<__nv_bfloat16*>(ws + pooled_ws_logits_bytes(BH, n));
@@ -672,13 +708,25 @@ extern "C" int moddit_pooled_map_ws(const float* qbar, const float* kbar, int BH
   split_means_kernel<<<dim3(static_cast<unsigned>((total4 + 255) / 256), 2), 256, 0, st>>>(
       qbar, kbar, nb, D, q_block_offset, k_block_offset, n, scale, total4, qs, ks);
   MODDIT_CHECK_LAUNCH("split_means_kernel");
-  pooled_logits_kernel<<<dim3(ceil_div(n, kLgCols), ceil_div(n, kLgRows), BH), kMapThreads, sm, st>>>(qs, ks, D, n, lg);
-  MODDIT_CHECK_LAUNCH("pooled_logits_kernel");
-  const int64_t rows = static_cast<int64_t>(BH) * n;
-  pooled_darkness_kernel<<<static_cast<unsigned>((rows + kMapThreads / 32 - 1) / (kMapThreads / 32)), kMapThreads, 0, st>>>(
-      lg, rows, n, static_cast<__half*>(map_f16));
-  MODDIT_CHECK_LAUNCH("pooled_darkness_kernel");
-  return MODDIT_OK;
+  return map_of_split_means(qs, ks, BH, D, n, lg, map_f16, st);
+}
+
+int moddit::pooled_map_of_blocks(const void* q, const void* k, int dtype, int BH, int N, int D, int block_size, int first, int n,
+                                 float scale, void* map_f16, void* workspace, cudaStream_t st) {
+  MODDIT_CHECK_ARG(q && k && map_f16, "pooled map: null pointer");
+  if (int rc = check_pool(q, dtype, BH, N, D, block_size)) return rc;
+  if (int rc = check_pool(k, dtype, BH, N, D, block_size)) return rc;
+  unsigned char* ws = static_cast<unsigned char*>(workspace);
+  float* lg = reinterpret_cast<float*>(ws);
+  PoolSplit split = {};
+  split.k = k;
+  split.qs = reinterpret_cast<__nv_bfloat16*>(ws + pooled_ws_logits_bytes(BH, n));
+  split.ks = reinterpret_cast<__nv_bfloat16*>(ws + pooled_ws_logits_bytes(BH, n) + pooled_ws_split_bytes(BH, n, D));
+  split.scale = scale;
+  split.first = first;
+  launch_pool<false, true>(q, dtype, D, N, block_size, nullptr, PoolShard{}, dim3(n, BH, 2), st, split);
+  MODDIT_CHECK_LAUNCH("pool_blocks_kernel (split)");
+  return map_of_split_means(split.qs, split.ks, BH, D, n, lg, map_f16, st);
 }
 
 // ---- strided row copy (used to place sequence/head shards directly into a peer GPU's buffer) ---------

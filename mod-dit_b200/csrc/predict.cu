@@ -1,7 +1,10 @@
 // Mask prediction of one denoising step in one call: block means of q and k, pooled map, line fit, features, line
-// selection, mask and work lists.  Nothing but the entry points of the single stages, one after the other on one
-// stream, with their scratch carved out of one workspace: a caller that goes through an interpreter pays for one call
-// and one scratch allocation instead of ten of each.  It matters where the stages themselves are a few microseconds each.
+// selection, mask and work lists: the single stages one after the other on one stream, with their scratch carved out of one
+// workspace, so that a caller that goes through an interpreter pays for one call and one scratch allocation instead of ten
+// of each.  It matters where the stages themselves are a few microseconds each.  Three launches of the single stages are
+// not made here: query and key are pooled together and their means leave split into the terms that the logits read, and
+// the solve writes its unknowns where the features go (a layer of four heads over 8,448 tokens 185 -> 172 us, of two heads
+// over 4,096 tokens 129 -> 120: launches and the gaps between them).
 #include "common.cuh"
 
 namespace moddit {
@@ -10,20 +13,17 @@ namespace {
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
 struct Scratch {
-  size_t qbar, kbar, map_ws, mts_ws, mts, solve_ws, X, selected, total;
+  size_t map_ws, mts_ws, mts, solve_ws, selected, total;
 };
 
-Scratch layout(int H, int nb, int D, int n, int top_k, bool small) {
+Scratch layout(int H, int D, int n, int top_k, bool small) {
   Scratch s = {};
   size_t at = 0;
   auto take = [&](size_t bytes) { const size_t p = at; at += up256(bytes); return p; };
-  s.qbar = take(sizeof(float) * static_cast<size_t>(H) * nb * D);
-  s.kbar = take(sizeof(float) * static_cast<size_t>(H) * nb * D);
   s.map_ws = take(moddit_pooled_map_workspace_bytes(H, n, D));
   s.mts_ws = take(moddit_mts_workspace_bytes(H, n));
   s.mts = take(sizeof(float) * static_cast<size_t>(H) * 3 * n);
   s.solve_ws = take(small ? 0 : moddit_solve_workspace_bytes(H, n));
-  s.X = take(sizeof(float) * static_cast<size_t>(H) * 3 * n);
   const int k = top_k < 3 * n - 1 ? top_k : 3 * n - 1;
   s.selected = take(sizeof(int64_t) * static_cast<size_t>(H) * (k > 0 ? k : 1));
   s.total = at;
@@ -37,7 +37,7 @@ using namespace moddit;
 
 extern "C" size_t moddit_predict_workspace_bytes(int H, int nb, int D, int n, int top_k, int small_solve) {
   if (H <= 0 || nb <= 0 || D <= 0 || n <= 0 || top_k <= 0) return 0;
-  return layout(H, nb, D, n, top_k, small_solve != 0).total;
+  return layout(H, D, n, top_k, small_solve != 0).total;
 }
 
 extern "C" int moddit_predict_lines(const void* q, const void* k, int dtype, int H, int N, int D, int block_size, int first,
@@ -65,31 +65,20 @@ extern "C" int moddit_predict_lines(const void* q, const void* k, int dtype, int
   } else {
     return fail(MODDIT_E_ARG, "predict_lines: unknown layout %d", mask_layout);
   }
-  const Scratch s = layout(H, nb, D, n, top_k, small_solve != 0);
+  const Scratch s = layout(H, D, n, top_k, small_solve != 0);
   if (workspace == nullptr || workspace_bytes < s.total || !aligned16(workspace))
     return fail(MODDIT_E_WORKSPACE, "predict_lines: %zu bytes of 16-byte aligned workspace needed", s.total);
   unsigned char* ws = static_cast<unsigned char*>(workspace);
-  float* qbar = reinterpret_cast<float*>(ws + s.qbar);
-  float* kbar = reinterpret_cast<float*>(ws + s.kbar);
   float* mts = reinterpret_cast<float*>(ws + s.mts);
-  float* X = reinterpret_cast<float*>(ws + s.X);
   int64_t* selected = reinterpret_cast<int64_t*>(ws + s.selected);
-  if (int rc = moddit_pool_blocks(q, dtype, H, N, D, block_size, qbar, stream)) return rc;
-  if (int rc = moddit_pool_blocks(k, dtype, H, N, D, block_size, kbar, stream)) return rc;
-  if (int rc = moddit_pooled_map_ws(qbar, kbar, H, nb, D, first, first, n, scale, map_f16, ws + s.map_ws,
-                                    moddit_pooled_map_workspace_bytes(H, n, D), stream))
+  if (int rc = pooled_map_of_blocks(q, k, dtype, H, N, D, block_size, first, n, scale, map_f16, ws + s.map_ws, as_stream(stream)))
     return rc;
   if (int rc = moddit_mts(map_f16, nullptr, nullptr, 0, 0, 0, nullptr, H, n, blocks_per_frame, mts, ws + s.mts_ws,
                           moddit_mts_workspace_bytes(H, n), stream))
     return rc;
-  if (small_solve) {
-    if (int rc = moddit_solve_small(mts, static_cast<const float*>(factor), H, n, X, stream)) return rc;
-  } else {
-    if (int rc = moddit_solve(mts, factor, H, n, blocks_per_frame, 1.0, X, ws + s.solve_ws,
+  if (int rc = solve_features(mts, factor, small_solve != 0, H, n, mode_threshold, d, c, b_d, modes, ws + s.solve_ws,
                               moddit_solve_workspace_bytes(H, n), stream))
-      return rc;
-  }
-  if (int rc = moddit_split_solution(X, H, n, mode_threshold, d, c, b_d, modes, stream)) return rc;
+    return rc;
   if (int rc = moddit_select_lines(c, d, last_c, last_d, H, n, top_k, predict_T, selected, stream)) return rc;
   const int chosen = top_k < 3 * n - 1 ? top_k : 3 * n - 1;
   const int text_blocks = mask_layout == MODDIT_LAYOUT_COGVIDEOX ? first : nb - n;

@@ -29,8 +29,8 @@ KERNELS_PER_CALL = {"moddit_pool_blocks": 1, "moddit_pooled_map": 1, "moddit_poo
                     "moddit_mtm": 1, "moddit_solve": 3, "moddit_select_lines": 1, "moddit_head_modes": 1,
                     "moddit_mask_from_lines": 1, "moddit_select_mass": 1, "moddit_tile_lists": 2,
                     "moddit_sparse_attn_fwd": 1, "moddit_replay_status": 0,
-                    # the stages of a prediction in one call: 2 + 3 + 2 + 3 (1 with the small solve) + 1 + 1 + 1 + 2
-                    "moddit_predict_lines": 15, "moddit_predict_lines (small)": 13,
+                    # the stages of a prediction in one call: 3 + 2 + 3 (1 with the small solve) + 1 + 1 + 2
+                    "moddit_predict_lines": 12, "moddit_predict_lines (small)": 10,
                     "moddit_mts_noalloc": 2, "moddit_copy_rows_dma": 0, "moddit_qkv_prologue": 1}
 
 
