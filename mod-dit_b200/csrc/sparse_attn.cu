@@ -89,12 +89,38 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
+// Which work item a block has.  The first 2 * n_single blocks have one query tile each, the two of a pair next to each other;
+// the others have a pair.
+struct BlockItem {
+  int npairs, item;
+  int flags;            // bits of its query tiles in a list entry: 0xff, 0x0f (the first only) or 0xf0 (the second only)
+  __device__ __forceinline__ BlockItem(int n_single, int Hm, const int32_t* order) {
+    const int b = static_cast<int>(blockIdx.x);
+    const bool single = b < 2 * n_single;
+    const int index = single ? b >> 1 : b - n_single;
+    npairs = (static_cast<int>(gridDim.x) - n_single) / Hm;
+    item = order ? order[index] : index;
+    flags = single ? ((b & 1) ? 0xf0 : 0x0f) : 0xff;
+  }
+};
+
+// Pairs whose two query tiles run as blocks of their own: as many as there would be idle SMs, the longest lists first (that is
+// how `order` begins).  A tile by itself has the exponential unit and the tensor pipe to itself; its rows are computed as in
+// a pair, bit for bit.  Launch alone: 132 pairs whose longest list is three times the mean 118 -> 108 us, 32 pairs at head
+// dimension 64 44 -> 38.
+int single_pairs(int items, int batches, int* n_single) {
+  int sms = 0;
+  if (int rc = sm_count(&sms)) return rc;
+  *n_single = min(items, max(0, sms / batches - items));
+  return MODDIT_OK;
+}
+
 template <int D, bool kBF16>
 __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
     const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
     const __grid_constant__ CUtensorMap tm_v, const int32_t* __restrict__ counts,
     const int32_t* __restrict__ entries, const int32_t* __restrict__ order, int Hm, int ntk, int N, float scale_log2, int q_split, int kvl_lo,
-    int kvl_hi, void* __restrict__ out_raw, float* __restrict__ lse, int32_t* __restrict__ status,
+    int kvl_hi, int n_single, void* __restrict__ out_raw, float* __restrict__ lse, int32_t* __restrict__ status,
     const __grid_constant__ OutScatter scatter) {
   constexpr int kTileBytes = kTile * D * 2;       // one Q, K or V tile
   constexpr int kChunks = D / 64;                 // 64-element (128-byte) column chunks per tile
@@ -114,15 +140,15 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
 
   const int warp = ptx::warp_index();
   const int lane = threadIdx.x % 32;
-  // grid: x = work item (mask head, query-tile pair), y = batch.  Blocks start in increasing blockIdx.x;
+  // grid: x = work item (mask head, query-tile pair, or one tile of it), y = batch.  Blocks start in increasing blockIdx.x;
   // `order` (from the work-list builder) puts long lists first, otherwise items run head by head.
-  const int npairs = static_cast<int>(gridDim.x) / Hm;
-  const int item = order ? order[blockIdx.x] : static_cast<int>(blockIdx.x);
+  const BlockItem blk(n_single, Hm, order);
+  const int npairs = blk.npairs, item = blk.item;
   const int mh = item / npairs;
   const int pair = item - mh * npairs;
   const int bh = blockIdx.y * Hm + mh;
   const int ntq = (N + kTile - 1) / kTile;
-  const bool has_b = (2 * pair + 1) < ntq;
+  if (2 * pair + (blk.flags == 0xf0) >= ntq) return;          // the second query tile of a pair that has one only
   const int cnt = counts[static_cast<int64_t>(mh) * npairs + pair];
   const int32_t* ent = entries + (static_cast<int64_t>(mh) * npairs + pair) * ntk;
 
@@ -153,8 +179,9 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (ptx::elect_one()) {
-      ptx::mbar_expect_tx(bar(kQFull), (has_b ? 2u : 1u) * kTileBytes);
-      for (int x = 0; x < (has_b ? 2 : 1); ++x)
+      const int q0 = blk.flags == 0xf0, q1 = blk.flags != 0x0f && 2 * pair + 1 < ntq;      // first and last query tile
+      ptx::mbar_expect_tx(bar(kQFull), (q1 - q0 + 1) * kTileBytes);
+      for (int x = q0; x <= q1; ++x)
         for (int c = 0; c < kChunks; ++c)
           ptx::tma_load_3d(sQ + x * kTileBytes + c * kChunkBytes, &tm_q, bar(kQFull), c * 64, (2 * pair + x) * kTile,
                            bh);
@@ -242,18 +269,18 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
         if (!ok) report(status, 2, 1, 0);
         if (ok) {
           ptx::tc_fence_after();
-          const int fl = ent[0] & 0xff;
+          const int fl = ent[0] & blk.flags;
           if (fl & 0x0f) issue_qk(0, 0);
           if (fl & 0xf0) issue_qk(1, 0);
           ptx::tc_commit(bar(kEmpty1));     // K stage 0 is free for the K tile of entry 2 (loaded with V of entry 1)
         }
       }
-      int fl_carry = (cnt > 0) ? (ent[0] & 0xff) : 0;
+      int fl_carry = (cnt > 0) ? (ent[0] & blk.flags) : 0;
       for (int e = 0; e < cnt && ok; ++e) {
         const int s = e & 1;
         const int fl = fl_carry;
         const bool next = (e + 1) < cnt;
-        const int fln = next ? (ent[e + 1] & 0xff) : 0;   // issued here, first used after the P V of tile A
+        const int fln = next ? (ent[e + 1] & blk.flags) : 0;   // issued here, first used after the P V of tile A
         fl_carry = fln;
         ok = ptx::mbar_wait(bar(kFull0 + s), (e >> 1) & 1, abort_flag);
         if (!ok) { report(status, 2, 1, e); break; }
@@ -283,6 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
     const int wq = warp % 4;                      // tensor-memory lane quarter of this warp
     const int r = wq * 32 + lane;                 // row inside the tile
     const int tile = 2 * pair + x;
+    const int mine = (blk.flags >> (4 * x)) & 0xf;      // 0: this block does not have the tile
     const int grow = tile * kTile + r;            // global query row
     const int kvl = (grow < q_split) ? kvl_lo : kvl_hi;
     const int kvl_min = min(kvl_lo, kvl_hi);
@@ -297,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
     bool ok = true;
     for (int e = 0; e < cnt; ++e) {
       const int en = ent[e];
-      const int sub = (en >> (4 * x)) & 0xf;
+      const int sub = (en >> (4 * x)) & mine;
       if (!sub) continue;
       const int col0 = (en >> 8) * kTile;
       ok = ptx::mbar_wait(bar(kSFullA + x), par_s, abort_flag);
@@ -398,7 +426,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
       ok = __all_sync(0xffffffffu, ok);
       if (!ok && lane == 0) report(status, 5, 2 + x, -1);
     }
-    if (ok && tile < ntq) {
+    if (ok && mine != 0 && tile < ntq) {
       ptx::tc_fence_after();
       const float inv = (done > 0 && l > 0.f) ? 1.f / l : 0.f;
       uint4* dst;
@@ -530,7 +558,7 @@ __global__ void __launch_bounds__(kThreads64, 1) sparse_attn_fwd_d64_kernel(
     const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
     const __grid_constant__ CUtensorMap tm_v, const int32_t* __restrict__ counts,
     const int32_t* __restrict__ entries, const int32_t* __restrict__ order, int Hm, int ntk, int N, float scale_log2,
-    int q_split, int kvl_lo, int kvl_hi, void* __restrict__ out_raw, float* __restrict__ lse,
+    int q_split, int kvl_lo, int kvl_hi, int n_single, void* __restrict__ out_raw, float* __restrict__ lse,
     int32_t* __restrict__ status, const __grid_constant__ OutScatter scatter) {
   constexpr int D = 64;
   constexpr int kTileBytes = kTile * D * 2;       // one Q, K or V tile: 128 rows x 128 bytes
@@ -550,13 +578,13 @@ __global__ void __launch_bounds__(kThreads64, 1) sparse_attn_fwd_d64_kernel(
 
   const int warp = ptx::warp_index();
   const int lane = threadIdx.x % 32;
-  const int npairs = static_cast<int>(gridDim.x) / Hm;
-  const int item = order ? order[blockIdx.x] : static_cast<int>(blockIdx.x);
+  const BlockItem blk(n_single, Hm, order);
+  const int npairs = blk.npairs, item = blk.item;
   const int mh = item / npairs;
   const int pair = item - mh * npairs;
   const int bh = blockIdx.y * Hm + mh;
   const int ntq = (N + kTile - 1) / kTile;
-  const bool has_b = (2 * pair + 1) < ntq;
+  if (2 * pair + (blk.flags == 0xf0) >= ntq) return;          // the second query tile of a pair that has one only
   const int cnt = counts[static_cast<int64_t>(mh) * npairs + pair];
   const int32_t* ent = entries + (static_cast<int64_t>(mh) * npairs + pair) * ntk;
 
@@ -590,8 +618,9 @@ __global__ void __launch_bounds__(kThreads64, 1) sparse_attn_fwd_d64_kernel(
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       if (ptx::elect_one()) {
-        ptx::mbar_expect_tx(bar(k6QFull), (has_b ? 2u : 1u) * kTileBytes);
-        for (int x = 0; x < (has_b ? 2 : 1); ++x)
+        const int q0 = blk.flags == 0xf0, q1 = blk.flags != 0x0f && 2 * pair + 1 < ntq;      // first and last query tile
+        ptx::mbar_expect_tx(bar(k6QFull), (q1 - q0 + 1) * kTileBytes);
+        for (int x = q0; x <= q1; ++x)
           ptx::tma_load_3d(sQ + x * kTileBytes, &tm_q, bar(k6QFull), 0, (2 * pair + x) * kTile, bh);
         bool ok = true;
         int issued = 0;
@@ -636,7 +665,7 @@ __global__ void __launch_bounds__(kThreads64, 1) sparse_attn_fwd_d64_kernel(
         };
         // the 64-key halves of an entry that the tile keeps in either half of its rows
         auto halves = [&](int e) -> uint32_t {
-          const uint32_t f = static_cast<uint32_t>(ent[e]) >> (4 * x);
+          const uint32_t f = static_cast<uint32_t>(ent[e] & blk.flags) >> (4 * x);
           return (f | (f >> 2)) & 3u;
         };
         auto issue_qk = [&](int h, int s) {   // s: K stage
@@ -706,7 +735,7 @@ __global__ void __launch_bounds__(kThreads64, 1) sparse_attn_fwd_d64_kernel(
     const uint32_t tS = tmem + lane_base + chain * 64;
     const uint32_t tO = tmem + lane_base + 256 + chain * 64;
     const int bit_mine = 4 * x + 2 * (r >> 6) + h;     // flag of this row half (the same for the whole warp)
-    const int bits_both = 0x5 << (4 * x + h);          // flags of this key half, both row halves
+    const int bits_both = (0x5 << (4 * x + h)) & blk.flags;   // flags of this key half, both row halves
 
     float m = -INFINITY, l = 0.f;
     uint32_t par_s = 0;
@@ -803,7 +832,7 @@ __global__ void __launch_bounds__(kThreads64, 1) sparse_attn_fwd_d64_kernel(
     }
     if (x == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
     else asm volatile("bar.sync 2, 256;" ::: "memory");
-    if (h == 0 && ok && tile < ntq) {
+    if (h == 0 && ok && bits_both != 0 && tile < ntq) {
       const float m1 = mg[64 * kTile + r], l1 = mg[65 * kTile + r];
       const float mm = fmaxf(m, m1);
       const float w0 = (m == -INFINITY) ? 0.f : ptx::ex2(m - mm);
@@ -872,8 +901,11 @@ int launch_d64(const void* q, const void* k, const void* v, int dtype, int BH, i
   const size_t smem = smem_bytes_d64();
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  kernel<<<dim3(npairs * Hm, BH / Hm), kThreads64, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N, scale_log2,
-                                                              q_split, kvl_lo, kvl_hi, out, lse, status, scatter);
+  int n_single = 0;
+  if (int rc = single_pairs(npairs * Hm, BH / Hm, &n_single)) return rc;
+  kernel<<<dim3(npairs * Hm + n_single, BH / Hm), kThreads64, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N,
+                                                                         scale_log2, q_split, kvl_lo, kvl_hi, n_single, out,
+                                                                         lse, status, scatter);
   MODDIT_CHECK_LAUNCH("sparse_attn_fwd_d64_kernel");
   return MODDIT_OK;
 }
@@ -892,8 +924,11 @@ int launch(const void* q, const void* k, const void* v, int dtype, int BH, int N
   const size_t smem = smem_bytes<D>();
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  kernel<<<dim3(npairs * Hm, BH / Hm), kThreads, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N, scale_log2, q_split,
-                                                   kvl_lo, kvl_hi, out, lse, status, scatter);
+  int n_single = 0;
+  if (int rc = single_pairs(npairs * Hm, BH / Hm, &n_single)) return rc;
+  kernel<<<dim3(npairs * Hm + n_single, BH / Hm), kThreads, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N,
+                                                                       scale_log2, q_split, kvl_lo, kvl_hi, n_single, out,
+                                                                       lse, status, scatter);
   MODDIT_CHECK_LAUNCH("sparse_attn_fwd_kernel");
   return MODDIT_OK;
 }
