@@ -354,6 +354,18 @@ int moddit_sparse_attn_fwd_scatter(const void* q, const void* k, const void* v, 
                                    void* const* peer_out, int n_peers, int head_base, float* lse,
                                    int32_t* status, void* stream);
 
+/* Either of the two (one of `out` and `peer_out` is null) as one of several launches that run at the same time on streams of
+ * their own, for instance one per group of heads.  `pairs_beside`: work items (Hm * npairs * batches) of the other launches.
+ * It decides nothing but how many pairs of query tiles run as two blocks; the output is the same bit for bit. */
+int moddit_sparse_attn_fwd_beside(const void* q, const void* k, const void* v, int dtype, int BH, int N, int D,
+                                  const int32_t* counts, const int32_t* entries, const int32_t* order, int Hm,
+                                  float softmax_scale, int q_split, int kv_len_lo, int kv_len_hi, int pairs_beside,
+                                  void* out, void* const* peer_out, int n_peers, int head_base, float* lse,
+                                  int32_t* status, void* stream);
+/* That number, for a launch of `pairs` = Hm * npairs pairs and `batches` batches on a GPU of `sms` SMs: idle SMs per batch,
+ * divided over the launches by their work items.  No GPU is needed. */
+int moddit_sparse_attn_single_pairs(int sms, int pairs, int batches, int pairs_beside);
+
 /* Attention prologue: the steps of the reference's attention processors between the q/k/v projections and the
  * attention call, in one pass (MoD/models/hunyuan/attention_processor.py:57-106: unflatten + transpose,
  * norm_q / norm_k, rotary embedding of the latent tokens, concatenation with the text stream;

@@ -236,6 +236,7 @@ def _engine_by_head_groups(query, key, value, lists, group_ready, scatter, **fwd
                                      lists.entries[h0:h1],
                                      order=flat_order[h0 * npairs:h1 * npairs].view(h1 - h0, npairs),
                                      check_status=False, out=None if out is None else out[:, h0:h1],
+                                     pairs_beside=(H - (h1 - h0)) * npairs,
                                      scatter=None if scatter is None else (scatter[0], scatter[1] + h0), **fwd_kw)
             done = torch.cuda.Event()
             done.record(st)

@@ -108,11 +108,13 @@ struct BlockItem {
 // how `order` begins).  A tile by itself has the exponential unit and the tensor pipe to itself; its rows are computed as in
 // a pair, bit for bit.  Launch alone: 132 pairs whose longest list is three times the mean 118 -> 108 us, 32 pairs at head
 // dimension 64 44 -> 38.
-int single_pairs(int items, int batches, int* n_single) {
-  int sms = 0;
-  if (int rc = sm_count(&sms)) return rc;
-  *n_single = min(items, max(0, sms / batches - items));
-  return MODDIT_OK;
+// Launches that run at the same time (`pairs_beside`: the others' work items) divide the idle SMs by their work items, because
+// a tile by itself needs more than half of its pair's time: two launches of 66 pairs take 74 us together (99 when each was
+// split as if it had the chip to itself, 81 without single tiles), three 120 (142, 123).
+int single_pairs(int sms, int items, int batches, int pairs_beside) {
+  const int64_t idle = max(0, (sms - pairs_beside) / batches - items);
+  const int64_t mine = static_cast<int64_t>(items) * batches;
+  return min(items, static_cast<int>(idle * mine / (mine + pairs_beside)));
 }
 
 template <int D, bool kBF16>
@@ -895,7 +897,7 @@ __global__ void __launch_bounds__(kThreads64, 1) sparse_attn_fwd_d64_kernel(
 template <bool kBF16>
 int launch_d64(const void* q, const void* k, const void* v, int dtype, int BH, int N, const int32_t* counts,
                const int32_t* entries, const int32_t* order, int Hm, float softmax_scale, int q_split, int kvl_lo,
-               int kvl_hi, void* out, float* lse, int32_t* status, const OutScatter& scatter, cudaStream_t st) {
+               int kvl_hi, int pairs_beside, void* out, float* lse, int32_t* status, const OutScatter& scatter, cudaStream_t st) {
   CUtensorMap tq, tk, tv;
   if (int rc = make_tmap_rows(&tq, q, dtype, BH, N, 64, kTile)) return rc;
   if (int rc = make_tmap_rows(&tk, k, dtype, BH, N, 64, kTile)) return rc;
@@ -906,8 +908,9 @@ int launch_d64(const void* q, const void* k, const void* v, int dtype, int BH, i
   const size_t smem = smem_bytes_d64();
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  int n_single = 0;
-  if (int rc = single_pairs(npairs * Hm, BH / Hm, &n_single)) return rc;
+  int sms = 0;
+  if (int rc = sm_count(&sms)) return rc;
+  const int n_single = single_pairs(sms, npairs * Hm, BH / Hm, pairs_beside);
   kernel<<<dim3(npairs * Hm + n_single, BH / Hm), kThreads64, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N,
                                                                          scale_log2, q_split, kvl_lo, kvl_hi, n_single, out,
                                                                          lse, status, scatter);
@@ -917,8 +920,8 @@ int launch_d64(const void* q, const void* k, const void* v, int dtype, int BH, i
 
 template <int D, bool kBF16>
 int launch(const void* q, const void* k, const void* v, int dtype, int BH, int N, const int32_t* counts,
-           const int32_t* entries, const int32_t* order, int Hm, float softmax_scale, int q_split, int kvl_lo, int kvl_hi, void* out,
-           float* lse, int32_t* status, const OutScatter& scatter, cudaStream_t st) {
+           const int32_t* entries, const int32_t* order, int Hm, float softmax_scale, int q_split, int kvl_lo, int kvl_hi,
+           int pairs_beside, void* out, float* lse, int32_t* status, const OutScatter& scatter, cudaStream_t st) {
   CUtensorMap tq, tk, tv;
   if (int rc = make_tmap_rows(&tq, q, dtype, BH, N, D, kTile)) return rc;
   if (int rc = make_tmap_rows(&tk, k, dtype, BH, N, D, kTile)) return rc;
@@ -929,8 +932,9 @@ int launch(const void* q, const void* k, const void* v, int dtype, int BH, int N
   const size_t smem = smem_bytes<D>();
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   const float scale_log2 = softmax_scale * 1.4426950408889634f;
-  int n_single = 0;
-  if (int rc = single_pairs(npairs * Hm, BH / Hm, &n_single)) return rc;
+  int sms = 0;
+  if (int rc = sm_count(&sms)) return rc;
+  const int n_single = single_pairs(sms, npairs * Hm, BH / Hm, pairs_beside);
   kernel<<<dim3(npairs * Hm + n_single, BH / Hm), kThreads, smem, st>>>(tq, tk, tv, counts, entries, order, Hm, ntq, N,
                                                                        scale_log2, q_split, kvl_lo, kvl_hi, n_single, out,
                                                                        lse, status, scatter);
@@ -943,10 +947,14 @@ int launch(const void* q, const void* k, const void* v, int dtype, int BH, int N
 
 using namespace moddit;
 
+extern "C" int moddit_sparse_attn_single_pairs(int sms, int pairs, int batches, int pairs_beside) {
+  return sms > 0 && pairs > 0 && batches > 0 && pairs_beside >= 0 ? single_pairs(sms, pairs, batches, pairs_beside) : 0;
+}
+
 static int sparse_attn_dispatch(const void* q, const void* k, const void* v, int dtype, int BH, int N, int D,
                                 const int32_t* counts, const int32_t* entries, const int32_t* order, int Hm,
-                                float softmax_scale, int q_split, int kv_len_lo, int kv_len_hi, void* out, float* lse,
-                                int32_t* status, const OutScatter& scatter, void* stream) {
+                                float softmax_scale, int q_split, int kv_len_lo, int kv_len_hi, int pairs_beside, void* out,
+                                float* lse, int32_t* status, const OutScatter& scatter, void* stream) {
   MODDIT_CHECK_ARG(q && k && v && counts && entries && status, "sparse_attn_fwd: null pointer");
   MODDIT_CHECK_ARG(out || scatter.n_peers > 0, "sparse_attn_fwd: no output destination");
   MODDIT_CHECK_ARG(BH > 0 && BH <= 65535 && N > 0 && Hm > 0, "sparse_attn_fwd: BH=%d N=%d Hm=%d out of range", BH, N, Hm);
@@ -954,6 +962,7 @@ static int sparse_attn_dispatch(const void* q, const void* k, const void* v, int
   MODDIT_CHECK_ARG(softmax_scale > 0.f, "sparse_attn_fwd: softmax_scale must be positive");
   MODDIT_CHECK_ARG(kv_len_lo >= 0 && kv_len_lo <= N && kv_len_hi >= 0 && kv_len_hi <= N,
                    "sparse_attn_fwd: kv_len (%d, %d) outside [0, N=%d]", kv_len_lo, kv_len_hi, N);
+  MODDIT_CHECK_ARG(pairs_beside >= 0, "sparse_attn_fwd: pairs_beside=%d must not be negative", pairs_beside);
   if (D != 64 && D != 128) return fail(MODDIT_E_UNSUPPORTED, "sparse_attn_fwd: head_dim must be 64 or 128, got %d", D);
   if (dtype != MODDIT_BF16 && dtype != MODDIT_FP16) return fail(MODDIT_E_ARG, "sparse_attn_fwd: unknown dtype %d", dtype);
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out))
@@ -963,14 +972,31 @@ static int sparse_attn_dispatch(const void* q, const void* k, const void* v, int
   if (D == 128) {
     return dtype == MODDIT_BF16
                ? launch<128, true>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                                   kv_len_hi, out, lse, status, scatter, st)
+                                   kv_len_hi, pairs_beside, out, lse, status, scatter, st)
                : launch<128, false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                                    kv_len_hi, out, lse, status, scatter, st);
+                                    kv_len_hi, pairs_beside, out, lse, status, scatter, st);
   }
-  return dtype == MODDIT_BF16 ? launch_d64<true>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
-                                                 kv_len_lo, kv_len_hi, out, lse, status, scatter, st)
-                              : launch_d64<false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split,
-                                                  kv_len_lo, kv_len_hi, out, lse, status, scatter, st);
+  return dtype == MODDIT_BF16
+             ? launch_d64<true>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo, kv_len_hi,
+                                pairs_beside, out, lse, status, scatter, st)
+             : launch_d64<false>(q, k, v, dtype, BH, N, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo, kv_len_hi,
+                                 pairs_beside, out, lse, status, scatter, st);
+}
+
+static int scatter_to(OutScatter* sc, void* const* peer_out, int n_peers, int N, int head_base) {
+  MODDIT_CHECK_ARG(peer_out, "sparse_attn_fwd_scatter: null peer table");
+  MODDIT_CHECK_ARG(n_peers >= 1 && n_peers <= kMaxPeers, "sparse_attn_fwd_scatter: n_peers=%d outside [1, %d]", n_peers,
+                   kMaxPeers);
+  MODDIT_CHECK_ARG(N % n_peers == 0, "sparse_attn_fwd_scatter: N=%d does not divide over %d peers", N, n_peers);
+  MODDIT_CHECK_ARG(head_base >= 0, "sparse_attn_fwd_scatter: head_base must be non-negative");
+  for (int i = 0; i < n_peers; ++i) {
+    MODDIT_CHECK_ARG(peer_out[i] && aligned16(peer_out[i]), "sparse_attn_fwd_scatter: peer buffer %d null or unaligned", i);
+    sc->peer[i] = peer_out[i];
+  }
+  sc->n_peers = n_peers;
+  sc->rows_per_peer = N / n_peers;
+  sc->head_base = head_base;
+  return MODDIT_OK;
 }
 
 extern "C" int moddit_sparse_attn_fwd(const void* q, const void* k, const void* v, int dtype, int BH, int N, int D,
@@ -979,9 +1005,8 @@ extern "C" int moddit_sparse_attn_fwd(const void* q, const void* k, const void* 
                                       float* lse, int32_t* status, void* stream) {
   clear_error();
   MODDIT_CHECK_ARG(out, "sparse_attn_fwd: null output pointer");
-  OutScatter none = {};
   return sparse_attn_dispatch(q, k, v, dtype, BH, N, D, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                              kv_len_hi, out, lse, status, none, stream);
+                              kv_len_hi, 0, out, lse, status, OutScatter{}, stream);
 }
 
 extern "C" int moddit_sparse_attn_fwd_scatter(const void* q, const void* k, const void* v, int dtype, int BH, int N,
@@ -990,19 +1015,22 @@ extern "C" int moddit_sparse_attn_fwd_scatter(const void* q, const void* k, cons
                                               int kv_len_lo, int kv_len_hi, void* const* peer_out, int n_peers,
                                               int head_base, float* lse, int32_t* status, void* stream) {
   clear_error();
-  MODDIT_CHECK_ARG(peer_out, "sparse_attn_fwd_scatter: null peer table");
-  MODDIT_CHECK_ARG(n_peers >= 1 && n_peers <= kMaxPeers, "sparse_attn_fwd_scatter: n_peers=%d outside [1, %d]", n_peers,
-                   kMaxPeers);
-  MODDIT_CHECK_ARG(N % n_peers == 0, "sparse_attn_fwd_scatter: N=%d does not divide over %d peers", N, n_peers);
-  MODDIT_CHECK_ARG(head_base >= 0, "sparse_attn_fwd_scatter: head_base must be non-negative");
   OutScatter sc = {};
-  for (int i = 0; i < n_peers; ++i) {
-    MODDIT_CHECK_ARG(peer_out[i] && aligned16(peer_out[i]), "sparse_attn_fwd_scatter: peer buffer %d null or unaligned", i);
-    sc.peer[i] = peer_out[i];
-  }
-  sc.n_peers = n_peers;
-  sc.rows_per_peer = N / n_peers;
-  sc.head_base = head_base;
+  if (int rc = scatter_to(&sc, peer_out, n_peers, N, head_base)) return rc;
   return sparse_attn_dispatch(q, k, v, dtype, BH, N, D, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
-                              kv_len_hi, nullptr, lse, status, sc, stream);
+                              kv_len_hi, 0, nullptr, lse, status, sc, stream);
+}
+
+extern "C" int moddit_sparse_attn_fwd_beside(const void* q, const void* k, const void* v, int dtype, int BH, int N, int D,
+                                             const int32_t* counts, const int32_t* entries, const int32_t* order, int Hm,
+                                             float softmax_scale, int q_split, int kv_len_lo, int kv_len_hi, int pairs_beside,
+                                             void* out, void* const* peer_out, int n_peers, int head_base, float* lse,
+                                             int32_t* status, void* stream) {
+  clear_error();
+  MODDIT_CHECK_ARG((out != nullptr) != (peer_out != nullptr), "sparse_attn_fwd_beside: one output destination, not both or none");
+  OutScatter sc = {};
+  if (peer_out != nullptr)
+    if (int rc = scatter_to(&sc, peer_out, n_peers, N, head_base)) return rc;
+  return sparse_attn_dispatch(q, k, v, dtype, BH, N, D, counts, entries, order, Hm, softmax_scale, q_split, kv_len_lo,
+                              kv_len_hi, pairs_beside, out, lse, status, sc, stream);
 }

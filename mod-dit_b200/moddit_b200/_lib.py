@@ -87,6 +87,10 @@ SIGNATURES = {
     "moddit_sparse_attn_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                        c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p,
                                        c_void_p, c_void_p]),
+    "moddit_sparse_attn_fwd_beside": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
+                                              c_void_p, c_void_p, c_int, c_float, c_int, c_int, c_int, c_int, c_void_p,
+                                              c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
+    "moddit_sparse_attn_single_pairs": (c_int, [c_int, c_int, c_int, c_int]),
 }
 
 for _name, (_res, _args) in SIGNATURES.items():

@@ -842,9 +842,11 @@ def sparse_attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, counts: t
                     softmax_scale: Optional[float] = None,
                     q_split: Optional[int] = None, kv_len_lo: Optional[int] = None,
                     kv_len_hi: Optional[int] = None, return_lse: bool = False, check_status=True,
-                    out: Optional[torch.Tensor] = None, scatter=None):
+                    out: Optional[torch.Tensor] = None, scatter=None, pairs_beside: int = 0):
     """Block-sparse attention forward of (B,H,N,D) tensors over the work lists from `tile_lists`.
 
+    pairs_beside: work items (mask heads x query-tile pairs x batches) of other launches that run at the same time on
+    other streams; same output, only the launch's shape takes them into account.
     check_status: True reads the kernel's status words after the launch (synchronises); "deferred" queues an
     asynchronous copy of them (`post_status`) for a later `check_posted_status`; False does neither."""
     dev = _need_cuda(q, k, v, counts, entries)
@@ -863,25 +865,25 @@ def sparse_attn_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, counts: t
     scale = float(D ** -0.5 if softmax_scale is None else softmax_scale)
     lse = torch.empty(B, H, N, device=dev, dtype=torch.float32) if return_lse else None
     st = _status_words(dev)
+    table, n_peers, head_base = None, 0, 0
     if scatter is not None:
         # scatter = (peer buffer pointers, head_base): output rows go straight into the peers' buffers
         peer_ptrs, head_base = scatter
-        table = (ctypes.c_void_p * len(peer_ptrs))(*peer_ptrs)
-        with torch.cuda.device(dev), _timed("moddit_sparse_attn_fwd", dev):
-            check(lib.moddit_sparse_attn_fwd_scatter(
-                _ptr(q), _ptr(k), _ptr(v), _qkv_dtype(q), B * H, N, D, _ptr(counts), _ptr(entries), _ptr(order), Hm,
-                scale, N if q_split is None else int(q_split), N if kv_len_lo is None else int(kv_len_lo),
-                N if kv_len_hi is None else int(kv_len_hi), table, len(peer_ptrs), int(head_base), _ptr(lse),
-                _ptr(st), _stream(dev)), "moddit_sparse_attn_fwd_scatter")
-        _after_launch(dev, check_status)
-        return (None, lse) if return_lse else None
-    if out is None:
+        table, n_peers = (ctypes.c_void_p * len(peer_ptrs))(*peer_ptrs), len(peer_ptrs)
+        out = None
+    elif out is None:
         out = torch.empty_like(q)
+    args = (_ptr(q), _ptr(k), _ptr(v), _qkv_dtype(q), B * H, N, D, _ptr(counts), _ptr(entries), _ptr(order), Hm, scale,
+            N if q_split is None else int(q_split), N if kv_len_lo is None else int(kv_len_lo),
+            N if kv_len_hi is None else int(kv_len_hi))
     with torch.cuda.device(dev), _timed("moddit_sparse_attn_fwd", dev):
-        check(lib.moddit_sparse_attn_fwd(_ptr(q), _ptr(k), _ptr(v), _qkv_dtype(q), B * H, N, D, _ptr(counts),
-                                         _ptr(entries), _ptr(order), Hm, scale, N if q_split is None else int(q_split),
-                                         N if kv_len_lo is None else int(kv_len_lo),
-                                         N if kv_len_hi is None else int(kv_len_hi), _ptr(out), _ptr(lse),
-                                         _ptr(st), _stream(dev)), "moddit_sparse_attn_fwd")
+        if pairs_beside:
+            check(lib.moddit_sparse_attn_fwd_beside(*args, int(pairs_beside), _ptr(out), table, n_peers, int(head_base),
+                                                    _ptr(lse), _ptr(st), _stream(dev)), "moddit_sparse_attn_fwd_beside")
+        elif scatter is not None:
+            check(lib.moddit_sparse_attn_fwd_scatter(*args, table, n_peers, int(head_base), _ptr(lse), _ptr(st),
+                                                     _stream(dev)), "moddit_sparse_attn_fwd_scatter")
+        else:
+            check(lib.moddit_sparse_attn_fwd(*args, _ptr(out), _ptr(lse), _ptr(st), _stream(dev)), "moddit_sparse_attn_fwd")
     _after_launch(dev, check_status)
     return (out, lse) if return_lse else out
