@@ -226,12 +226,16 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
     if (ptx::elect_one()) {
       // Descriptor bases are built once; inside the loops an MMA costs one 32-bit add per operand (the
       // issuing thread shares its scheduler with two busy softmax warps, so every instruction counts).
-      const uint64_t dq0 = ptx::smem_desc_sw128(sQ, 16, 1024), dk0 = ptx::smem_desc_sw128(sK, 16, 1024);
-      const uint64_t dv0 = ptx::smem_desc_sw128(sV, kChunkBytes, 1024);
       auto advance = [](uint64_t desc, uint32_t bytes) -> uint64_t {
         // the start-address field (bits 0-13, units of 16 bytes) never carries out for shared-memory addresses
         return (desc & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(desc) + (bytes >> 4));
       };
+      // Registers are short here (72): K's descriptor is derived from Q's, the per-tile state is bits of one word, and nothing
+      // is kept to remember an early Q K^T by.  With a bit mask per tile and both tiles' products in either place 12 bytes
+      // were spilled inside the loop, which cost launches without one-sided entries 1 - 1.5 % (492 pairs, 4 % one-sided:
+      // 166 -> 169 us, now 167).
+      const uint64_t dq0 = ptx::smem_desc_sw128(sQ, 16, 1024), dk0 = advance(dq0, sK - sQ);
+      const uint64_t dv0 = ptx::smem_desc_sw128(sV, kChunkBytes, 1024);
       auto issue_qk = [&](int x, int s) {
         const uint64_t a0 = advance(dq0, x * kTileBytes), b0 = advance(dk0, s * kTileBytes);
         const uint32_t d = tmem + x * 128;
@@ -264,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
       };
       bool ok = ptx::mbar_wait(bar(kQFull), 0, abort_flag);
       if (!ok) report(status, 2, 1, -1);
-      uint32_t par_p = 0, acc = 0;          // a bit per tile
+      uint32_t tiles = 0;                   // bit x: parity of tile x's P, bit 2 + x: tile x has an accumulator
       if (ok && cnt > 0) {
         ok = ptx::mbar_wait(bar(kKFirst), 0, abort_flag);
         if (!ok) report(status, 2, 1, 0);
@@ -285,22 +289,23 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
         fl_carry = fln;
         ok = ptx::mbar_wait(bar(kFull0 + s), (e >> 1) & 1, abort_flag);
         if (!ok) { report(status, 2, 1, e); break; }
-        // A tile that does not keep this entry starts on the next one before the other tile's P is waited for: where two
-        // neighbouring entries are kept by one tile each (a diagonal does that), both tiles work at the same time (launches
-        // with 24 - 50 % of such entries 1.5 - 3 % shorter, others the same).
-#pragma unroll
-        for (int x = 0; x < 2; ++x)
-          if (!(fl & (0xf << (4 * x))) && (fln & (0xf << (4 * x)))) issue_qk(x, s ^ 1);
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          if (!(fl & (0xf << (4 * x)))) continue;
-          ok = pv_when_ready(x, s, (acc >> x) & 1u, (par_p >> x) & 1u);
+        // A tile that does not keep this entry starts on the next one before the other tile's P is waited for (tile A does so
+        // by its place): where neighbouring entries are kept by one tile each (a diagonal does that), both tiles work at the
+        // same time.  Launches with 20 - 50 % of such entries take 1 - 4 % less (Wan's layer 15.54 -> 15.21 ms, the
+        // cumulative-mass clip 685 -> 669 us), the others the same.
+        if (!(fl & 0xf0) && (fln & 0xf0)) issue_qk(1, s ^ 1);
+        if (fl & 0x0f) {
+          ok = pv_when_ready(0, s, tiles & 4u, tiles & 1u);
           if (!ok) { report(status, 3, 1, e); break; }
-          par_p ^= 1u << x;
-          acc |= 1u << x;
-          if (fln & (0xf << (4 * x))) issue_qk(x, s ^ 1);
+          tiles = (tiles ^ 1u) | 4u;
         }
-        if (!ok) break;
+        if (fln & 0x0f) issue_qk(0, s ^ 1);
+        if (fl & 0xf0) {
+          ok = pv_when_ready(1, s, tiles & 8u, (tiles >> 1) & 1u);
+          if (!ok) { report(status, 3, 1, e); break; }
+          tiles = (tiles ^ 2u) | 8u;
+          if (fln & 0xf0) issue_qk(1, s ^ 1);
+        }
         ptx::tc_commit(bar(kEmpty0 + s));
       }
       ptx::tc_commit(bar(kOFinal));
