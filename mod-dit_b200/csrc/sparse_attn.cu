@@ -230,10 +230,6 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
         // the start-address field (bits 0-13, units of 16 bytes) never carries out for shared-memory addresses
         return (desc & 0xffffffff00000000ull) | static_cast<uint32_t>(static_cast<uint32_t>(desc) + (bytes >> 4));
       };
-      // Registers are short here (72): K's descriptor is derived from Q's, the per-tile state is bits of one word, and nothing
-      // is kept to remember an early Q K^T by.  With a bit mask per tile and both tiles' products in either place 12 bytes
-      // were spilled inside the loop, which cost launches without one-sided entries 1 - 1.5 % (492 pairs, 4 % one-sided:
-      // 166 -> 169 us, now 167).
       const uint64_t dq0 = ptx::smem_desc_sw128(sQ, 16, 1024), dk0 = advance(dq0, sK - sQ);
       const uint64_t dv0 = ptx::smem_desc_sw128(sV, kChunkBytes, 1024);
       auto issue_qk = [&](int x, int s) {
@@ -289,23 +285,24 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
         fl_carry = fln;
         ok = ptx::mbar_wait(bar(kFull0 + s), (e >> 1) & 1, abort_flag);
         if (!ok) { report(status, 2, 1, e); break; }
-        // A tile that does not keep this entry starts on the next one before the other tile's P is waited for (tile A does so
-        // by its place): where neighbouring entries are kept by one tile each (a diagonal does that), both tiles work at the
-        // same time.  Launches with 20 - 50 % of such entries take 1 - 4 % less (Wan's layer 15.54 -> 15.21 ms, the
-        // cumulative-mass clip 685 -> 669 us), the others the same.
-        if (!(fl & 0xf0) && (fln & 0xf0)) issue_qk(1, s ^ 1);
-        if (fl & 0x0f) {
-          ok = pv_when_ready(0, s, tiles & 4u, tiles & 1u);
-          if (!ok) { report(status, 3, 1, e); break; }
-          tiles = (tiles ^ 1u) | 4u;
-        }
-        if (fln & 0x0f) issue_qk(0, s ^ 1);
-        if (fl & 0xf0) {
-          ok = pv_when_ready(1, s, tiles & 8u, (tiles >> 1) & 1u);
-          if (!ok) { report(status, 3, 1, e); break; }
-          tiles = (tiles ^ 2u) | 8u;
-          if (fln & 0xf0) issue_qk(1, s ^ 1);
-        }
+        // A tile that does not keep this entry starts on the next one before the other tile's P is waited for: where two
+        // neighbouring entries are kept by one tile each (a diagonal does that), both tiles work at the same time.  So the
+        // slot begins with the second tile where that has no P V; the tile's number is a run-time value, because the copies
+        // of the products that constants need cost launches without such entries more than they gain.  Launch, fixed order /
+        // one copy for either tile here and a further one for the early scores / this: dense 24 heads x 6,820 tokens 542 /
+        // 540 - 549 / 525 us, HunyuanVideo (12 % one-sided) 21.06 / 20.89 / 20.41 ms, Wan (21 %) 15.54 / 15.23 / 14.94,
+        // cumulative-mass clip (50 %) 693 / 677 / 669 us; one copy in a loop of two 536, 20.87, 15.31, 677.
+        const int first = (fl & 0xf0) ? 0 : 1;
+        auto half_slot = [&](int x) -> bool {
+          if ((fl >> (4 * x)) & 0xf) {
+            if (!pv_when_ready(x, s, tiles & (4u << x), (tiles >> x) & 1u)) return false;
+            tiles = (tiles ^ (1u << x)) | (4u << x);
+          }
+          if ((fln >> (4 * x)) & 0xf) issue_qk(x, s ^ 1);
+          return true;
+        };
+        ok = half_slot(first) && half_slot(first ^ 1);
+        if (!ok) { report(status, 3, 1, e); break; }
         ptx::tc_commit(bar(kEmpty0 + s));
       }
       ptx::tc_commit(bar(kOFinal));
