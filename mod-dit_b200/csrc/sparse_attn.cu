@@ -3,7 +3,9 @@
 // warp-specialised online softmax.
 //
 // One CTA owns a PAIR of adjacent 128-row query tiles (A, B) of one head and walks the union of
-// their key-tile lists, so a K/V tile needed by both is fetched once.  Roles (12 warps):
+// their key-tile lists, so a K/V tile needed by both is fetched once.  Where a launch has fewer pairs than
+// SMs a CTA may own one tile of a pair; it walks the same list and passes over what the tile does not keep.
+// Roles (12 warps):
 //   warp 0      TMA producer: Q tiles once, then K and V tiles through two 2-stage rings (V of entry e and K
 //               of entry e + 1 share their barriers: they are consumed together)
 //   warp 1      MMA issuer: S_X = Q_X K^T (SS form), O_X += P_X V (P read from tensor memory)
@@ -13,8 +15,10 @@
 // Tensor memory (512 columns): S_A [0,128) S_B [128,256) O_A [256,256+D) O_B [256+D,256+2D); P_X
 // (16-bit) overwrites the first 64 columns of S_X.  MMAs issued by one thread execute in order, which
 // is what makes the aliasing and the "S ready implies the previous P V finished" reasoning valid.
-// The issue order  PV(A,e) QK(A,e+1) PV(B,e) QK(B,e+1)  lets the softmax of one tile overlap the MMAs
-// of the other.
+// The issue order of an entry that both tiles keep,  PV(A,e) QK(A,e+1) PV(B,e) QK(B,e+1),  lets the softmax
+// of one tile overlap the MMAs of the other.  A tile that does not keep entry e has no P V in it, so its
+// QK(e+1) comes first (B's before A's part if need be): the tile's last P V was issued earlier by the same
+// thread, and K(e+1) has landed with V(e), which was waited for.
 //
 // Every wait is bounded (ptx::mbar_wait); on expiry the CTA records a status word, lets its copies
 // land, releases tensor memory and returns.
@@ -104,10 +108,11 @@ struct BlockItem {
   }
 };
 
-// Pairs whose two query tiles run as blocks of their own: as many as there would be idle SMs, the longest lists first (that is
-// how `order` begins).  A tile by itself has the exponential unit and the tensor pipe to itself; its rows are computed as in
-// a pair, bit for bit.  Launch alone: 132 pairs whose longest list is three times the mean 118 -> 108 us, 32 pairs at head
-// dimension 64 44 -> 38.
+// Pairs whose two query tiles run as blocks of their own: as many as there would be idle SMs, the first ones of `order` (the two
+// longest lists of every head, then the first head's from the longest on, the second head's, ...; without an order the first
+// by index).  A tile by itself has the exponential unit and the tensor pipe to itself; its rows are computed as in a pair, bit
+// for bit.  It fetches K and V of the whole list of its pair, also of entries that only the other tile keeps.  Launch alone:
+// 132 pairs whose longest list is three times the mean 118 -> 108 us, 32 pairs at head dimension 64 44 -> 38.
 // Launches that run at the same time (`pairs_beside`: the others' work items) divide the idle SMs by their work items, because
 // a tile by itself needs more than half of its pair's time: two launches of 66 pairs take 74 us together (99 when each was
 // split as if it had the chip to itself, 81 without single tiles), three 120 (142, 123).
@@ -172,8 +177,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
   const uint32_t tmem = ctl->tmem_base;
 
   // Register budget: the softmax warpgroups hold a 128-value row per thread, the control warps need little
-  // (128 control threads give up what 256 softmax threads take: 168 -> 72 / 216, the split that leaves each
-  // instantiation without a spill).
+  // (128 control threads give up what 256 softmax threads take: 168 -> 72 / 216, the split that spills least).
   // The control branch and the softmax branch are disjoint in the control-flow graph so that each gets
   // its own register allocation.
   if (warp < 4) {
@@ -492,14 +496,16 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn_fwd_kernel(
 // exchanged until the two accumulators of a row are put together at the end.
 //   S_c [64 c, 64 c + 64)   O_c [256 + 64 c, 320 + 64 c)   for chain c = 2 * tile + half; P_c (16-bit) overwrites the first
 //   32 columns of S_c.
-// Each query tile has an issuing thread that takes its two chains in turn, PV(0,e) QK(0,e+1) PV(1,e) QK(1,e+1): products of
-// one thread execute in order, which makes the aliasing of P and S safe and lets "S ready" imply that the chain's previous
-// P V is done.  A half that neither half of the tile's rows keeps costs nothing.
-// Measured, launch alone, before -> now: 48 heads x 45,104 tokens at 12 % of the blocks 4.82 -> 4.22 ms, 32 heads x 16,640
-// tokens at 33 % 1.21 -> 1.07, dense 48 heads x 20,624 tokens 7.2 -> 6.1-6.4.
+// Each query tile has an issuing thread that takes its two chains in turn, PV(0,e) QK(0,e+1) PV(1,e) QK(1,e+1); a chain that
+// entry e does not concern has its QK(e+1) first.  Products of one thread execute in order, which makes the aliasing of P and
+// S safe and lets "S ready" imply that the chain's previous P V is done.  A half that neither half of the tile's rows keeps
+// costs nothing.
+// Measured, launch alone, before -> now, in turn in one process: 48 heads x 45,104 tokens at 12 % of the blocks 4.87 -> 4.19
+// ms, 32 heads x 16,640 tokens at 33 % 1.22 -> 1.08, dense 48 heads x 20,624 tokens 7.29 -> 6.17 (7.35 -> 6.65 where the power
+// limit holds the clock down after a second of such launches).
 // ====================================================================================================
 constexpr int kThreads64 = 640;   // 4 control warps, 4 softmax warpgroups
-constexpr int kStages64 = 3;      // K and V tiles in flight (16 KB each)
+constexpr int kStages64 = 3;      // K and V tiles in flight (16 KB each); four would not fit beside the merge buffer
 enum BarrierIndex64 {
   k6QFull = 0,
   k6KFirst,
